@@ -266,10 +266,10 @@ cudaError_t launch_large(const MatrixF32& M, const SetSource& src, const SetOutp
   return cudaGetLastError();
 }
 
-template <int KB, int CS, int NTC, int RPT = 1>
+template <int KB, int CS, int NTC, int RPT = 1, int AF = 0>
 cudaError_t launch_cluster(const MatrixF32& M, const SetSource& src, const SetOutputs& out,
                            long long nitems, void*, cudaStream_t st, bool prep) {
-  auto kern = k_cluster_solve<KB, CS, NTC, RPT>;
+  auto kern = k_cluster_solve<KB, CS, NTC, RPT, AF>;
   const size_t dsm = sizeof(ClusterSmem<KB, CS, NTC>);
   static int maxcl = [&] {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm);
@@ -376,11 +376,12 @@ struct Variant {
     "cluster KB=" #KB " CS=" #CS " NTC=" #NTC,                                                  \
         {launch_cluster<KB, CS, NTC>, nullptr}, {scratch_none, scratch_none}                    \
   }
-// RPT rows per thread (each with KB / TPR columns of P)
-#define CLUSTERR(KB, CS, NTC, RPT)                                                            \
+// RPT rows per thread (each with KB / TPR columns of P), AF chunks of A's rows
+// read ahead per step
+#define CLUSTERR(KB, CS, NTC, RPT, AF)                                                            \
   Variant {                                                                                     \
     "cluster KB=" #KB " CS=" #CS " NTC=" #NTC " RPT=" #RPT,                                     \
-        {launch_cluster<KB, CS, NTC, RPT>, nullptr}, {scratch_none, scratch_none}               \
+        {launch_cluster<KB, CS, NTC, RPT, AF>, nullptr}, {scratch_none, scratch_none}           \
   }
 // upper 32 x 32 tiles of A_S and P, one set per CTA (NB blocks of 32, NW warps of TPW tiles)
 #define SYM(NB, NW, TPW, MINB)                                                                 \
@@ -410,14 +411,14 @@ const std::vector<Variant>& variants(int b) {
       {SA(128, 1, 128, 3), REG(128, 1, 2, 256, 1), SA(128, 1, 128, 2), SA2(128, 128, 2), SYM(4, 5, 2, 3),
        SYM(4, 10, 1, 2)},
       {CLUSTER(192, 2, 384), LARGE(256), CLUSTER(192, 4, 192), CLUSTER(192, 1, 384), CLUSTER(192, 1, 768),
-       CLUSTERR(192, 1, 384, 2), CLUSTERR(192, 1, 384, 4), SYM(6, 11, 2, 1), SYM(6, 21, 1, 1),
+       CLUSTERR(192, 1, 384, 2, 0), CLUSTERR(192, 1, 384, 4, 0), SYM(6, 11, 2, 1), SYM(6, 21, 1, 1),
        SYM(6, 16, 2, 1)},
       {CLUSTER(256, 2, 512), LARGE(256), CLUSTER(256, 4, 256), CLUSTER(256, 8, 256), CLUSTER(256, 2, 256),
-       CLUSTERR(256, 2, 256, 2), CLUSTERR(256, 2, 256, 4), SYM(8, 12, 3, 1)},
-      {CLUSTER(384, 4, 384), LARGE(512), CLUSTER(384, 8, 192), CLUSTER(384, 6, 256), CLUSTERR(384, 6, 256, 2),
-       CLUSTERR(384, 6, 256, 4), CLUSTERR(384, 4, 384, 4)},
-      {CLUSTER(512, 8, 256), LARGE(512), CLUSTER(512, 8, 512), CLUSTERR(512, 8, 256, 2),
-       CLUSTERR(512, 8, 256, 4)},
+       CLUSTERR(256, 2, 256, 2, 0), CLUSTERR(256, 2, 256, 4, 0), SYM(8, 12, 3, 1)},
+      {CLUSTER(384, 4, 384), LARGE(512), CLUSTER(384, 8, 192), CLUSTER(384, 6, 256), CLUSTERR(384, 6, 256, 2, 0),
+       CLUSTERR(384, 6, 256, 4, 4), CLUSTERR(384, 4, 384, 4, 2)},
+      {CLUSTER(512, 8, 256), LARGE(512), CLUSTER(512, 8, 512), CLUSTERR(512, 8, 256, 2, 5),
+       CLUSTERR(512, 8, 256, 4, 0)},
   };
   return v[b];
 }

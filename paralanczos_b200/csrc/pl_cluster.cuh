@@ -7,32 +7,50 @@
 // its rows of P in registers.  Same recurrence as pl_engine.cuh (three-term
 // step, w = P w~, P -= v v^T fused with the next matvec, FP32 vectors, FP64
 // alpha/beta).  Per step the CTAs exchange, through distributed shared memory:
-// their FP64 partials of alpha and ||w||^2 (every CTA sums the CS partials in
-// rank order, so the scalars are bitwise identical cluster-wide and every
-// branch is cluster-uniform), and their rows of w~ and w (written into every
-// peer's broadcast buffers).  Two cluster barriers per step: one carries the
-// rows of y = A v with the alpha partials (each CTA then forms all of
-// w~ = y - alpha v_j - beta_j v_{j-1} locally), one carries the rows of w with
-// the ||w||^2 partials.
+// their FP64 partials of alpha and ||w||^2 (one per warp; every warp adds all
+// of them in the same order, so the scalars are bitwise identical cluster-wide
+// and every branch is cluster-uniform), and their rows of y = A v and w
+// (written into every peer's broadcast buffers).
+//
+// What bounds it is the latency of the two exchanges of a step, so they are
+// built to be short: each lane that holds a finished row sum writes it into
+// the peers with st.async, whose bytes the receiving CTA's mbarrier counts;
+// a warp sends as soon as its rows are done and waits only for the bytes it
+// needs.  No CTA barrier, no cluster barrier (whose release fence the warps
+// would wait for) and no second pass over the partials.  Measured with a
+// cluster barrier per exchange and then with st.async (B200, sets/s): k = 384
+// (1,000 sets) 2.55e4 -> 3.39e4, k = 512 (600 sets) 8.7e3 -> 1.19e4, and with
+// the same reductions inside one CTA k = 192 (3,000 sets) 3.06e5 -> 3.55e5.
 //
 // Thread mapping inside a CTA: NTC threads; a thread holds RPT of the CTA's
 // R rows (rows ls, ls + R/RPT, ...), TPR = NTC * RPT / R threads share a row;
-// thread g = t % TPR of a row owns the float4 column chunks g, g + TPR,
-// g + 2 TPR, ... (CPT = KB / TPR columns of each of its rows), so the TPR
-// threads of a row read adjacent 16-byte chunks of a broadcast vector:
-// conflict-free shared-memory loads.  Row partial sums are combined with
-// xor-shuffles over the TPR lanes (TPR divides 32).  With RPT = 2 a thread
-// holds as much of P as with one row of twice the columns, but reads half of
-// each broadcast vector per step.
+// thread g of a row owns the float4 column chunks g, g + TPR, g + 2 TPR, ...
+// (CPT = KB / TPR columns of each of its rows).  The lanes of one g are
+// adjacent in the warp: a 128-bit load of a broadcast vector in which
+// neighbouring lanes share an address takes 2.1 cycles of the shared-memory
+// pipe, one in which they do not takes 4.0 whatever else is shared (measured),
+// and these loads are a third of the pipe's work.  Row partial sums are combined with
+// xor-shuffles over the TPR lanes (TPR divides 32): the first log2(RPT) levels
+// halve the rows each lane goes on with (a lane sends the half it drops), so
+// TPR / RPT lanes end with each row's sum, one per peer to send it to.  With
+// RPT = 2 a thread holds as much of P as with one row of twice the columns,
+// but reads half of each broadcast vector per step.
 #pragma once
 #include <cooperative_groups.h>
 
 #include "pl_engine.cuh"
 #include "pl_sturm.cuh"
+#include "pl_sync.cuh"
 
 namespace pl {
 
 namespace cg = cooperative_groups;
+
+__host__ __device__ constexpr int pow2_up(int n) {
+  int p = 1;
+  while (p < n) p *= 2;
+  return p;
+}
 
 template <int KB, int CS, int NTC, int RPT = 1>
 struct CfgC {
@@ -43,22 +61,54 @@ struct CfgC {
   static constexpr int NCH = CPT / 4;     // float4 chunks per thread and row
   static constexpr int NWC = NTC / 32;    // warps per CTA
   static_assert(KB % CS == 0 && R % RPT == 0 && NTC % RS == 0 && KB % TPR == 0, "bad shape");
+  static constexpr int CPR = TPR / RPT;  // lanes that end with a row's sum
+  static constexpr int NP = (CS + CPR - 1) / CPR;  // peers such a lane sends it to
   static_assert(32 % TPR == 0 && CPT % 4 == 0, "bad shape");
+  static_assert(TPR % RPT == 0 && (RPT & (RPT - 1)) == 0 && CS <= 32, "bad shape");
 };
 
 template <int KB, int CS, int NTC>
 struct __align__(16) ClusterSmem {
+  static constexpr int NPART = CS * (NTC / 32);  // one partial per warp of the set
   float4 A[(KB / CS) * KB / 4];  // own rows, [chunk][thread]
   float vb[3][KB];               // unnormalised Lanczos vectors, rotating: current, previous, next
   float yb[KB];                  // broadcast of y = A v
   float wb[KB];                  // w~, formed locally from yb
   int idx[KB];
   double2 ab[KB];                // T (rank 0 reads it for the bisection)
-  double part[4][CS > NTC / 32 ? CS : NTC / 32];  // alpha, ||w||^2, misc, index check: rank
-                                                // partials (warp partials for one CTA)
-  double red[NTC / 32];          // warp partials inside the CTA
+  double part[4][NPART];         // alpha, ||w||^2, misc, index check
+  double ext[2];                 // lambda_min, lambda_max
+  double red[NTC / 32];          // warp partials inside the CTA (breakdown argmax)
   unsigned long long key[CS];    // breakdown argmax exchange
+  unsigned long long bar[2];     // mbarriers of the y and the w exchange
+  int abort;                     // a bounded wait gave up
 };
+
+// What one exchange delivers into every CTA: KB rows and the warps' partials.
+template <int KB, int CS, int NTC>
+__device__ __forceinline__ constexpr uint32_t exchange_bytes() {
+  return KB * sizeof(float) + ClusterSmem<KB, CS, NTC>::NPART * sizeof(double);
+}
+
+// Address of this CTA's shared-memory address `a` in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t peer_addr(uint32_t a, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void st_async(uint32_t a, float x, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(a),
+               "r"(__float_as_uint(x)), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void st_async(uint32_t a, double x, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(a),
+               "l"(__double_as_longlong(x)), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
 
 // Barrier over the set's CTAs.  A one-CTA cluster needs only the CTA barrier
 // (same ordering of its shared-memory writes, without the cluster-scope
@@ -71,58 +121,112 @@ __device__ __forceinline__ void set_sync(cg::cluster_group& cl) {
     cl.sync();
 }
 
-// Sum over the CTA, then over the cluster (rank order).  Identical everywhere.
-// A one-CTA set skips the CTA-level step: each warp's lane 0 stores its
-// partial in part[slot][warp], one block barrier, and every thread adds the
-// warps' partials in warp order.  (With several CTAs per set, the same scheme
-// -- every warp storing into every peer -- measured slower than one CTA
-// barrier plus one store per peer.)
+// Sum of the N partials of an exchange by one warp (the same order in every
+// warp of every CTA).
+template <int N>
+__device__ __forceinline__ double part_sum(const double* p) {
+  const int lane = threadIdx.x & 31;
+  double s = lane < N ? p[lane] : 0.0;
+#pragma unroll
+  for (int i = 32; i < N; i += 32)
+    if (i + lane < N) s += p[i + lane];
+  return warp_sum(s);
+}
+
+// Sum over the set's CTAs outside the step loop (cluster barrier).
 template <int KB, int CS, int NTC>
 __device__ __forceinline__ double cluster_sum(double x, ClusterSmem<KB, CS, NTC>& sm, int slot,
                                               cg::cluster_group& cl, int rank) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-  const int w = threadIdx.x >> 5;
-  if constexpr (CS == 1) {
-    if ((threadIdx.x & 31) == 0) sm.part[slot][w] = x;
-    __syncthreads();
-    double s = sm.part[slot][0];
-#pragma unroll
-    for (int i = 1; i < NTC / 32; ++i) s += sm.part[slot][i];
-    return s;
-  } else {
-    if ((threadIdx.x & 31) == 0) sm.red[w] = x;
-    __syncthreads();
-    if (threadIdx.x < CS) {
-      double s = sm.red[0];
-#pragma unroll
-      for (int i = 1; i < NTC / 32; ++i) s += sm.red[i];
-      ClusterSmem<KB, CS, NTC>* peer = cl.map_shared_rank(&sm, (unsigned)threadIdx.x);
-      peer->part[slot][rank] = s;
-    }
-    set_sync<CS>(cl);
-    double s = sm.part[slot][0];
-#pragma unroll
-    for (int r = 1; r < CS; ++r) s += sm.part[slot][r];
-    return s;
+  const double s = warp_sum(x);
+  const int lane = threadIdx.x & 31;
+  if (lane < CS) {
+    ClusterSmem<KB, CS, NTC>* peer = CS == 1 ? &sm : cl.map_shared_rank(&sm, (unsigned)lane);
+    peer->part[slot][rank * (NTC / 32) + (threadIdx.x >> 5)] = s;
   }
+  set_sync<CS>(cl);
+  return part_sum<ClusterSmem<KB, CS, NTC>::NPART>(sm.part[slot]);
 }
 
-template <int KB, int CS, int NTC, int RPT = 1>
-__device__ __forceinline__ void cluster_solve_set(const MatrixF32& M, const int* __restrict__ S,
+// Row sums of a thread's RPT rows over the row's TPR lanes: the xor tree
+// TPR/2, ..., 1, each level down to one row dropping half of the rows.  Lane
+// g0 ends with the sum of row g0 / (TPR / RPT).
+template <int RPT, int TPR>
+__device__ __forceinline__ float row_reduce(float (&y)[RPT], int g0) {
+  constexpr int RPW = 32 / TPR;  // lanes of one g (adjacent)
+  int n = RPT;
+#pragma unroll
+  for (int o = TPR / 2; o > 0; o >>= 1) {
+    if (n > 1) {
+      n /= 2;
+      const bool hi = g0 & o;
+#pragma unroll
+      for (int e = 0; e < RPT / 2; ++e)
+        if (e < n) {
+          const float keep = hi ? y[e + n] : y[e], send = hi ? y[e] : y[e + n];
+          y[e] = keep + __shfl_xor_sync(0xffffffffu, send, o * RPW);
+        }
+    } else {
+      y[0] += __shfl_xor_sync(0xffffffffu, y[0], o * RPW);
+    }
+  }
+  return y[0];
+}
+
+// Solves one set on the cluster.  false: a bounded wait gave up (the set is
+// reported as failed and the kernel must end).  ph: phase parity of the
+// exchanges, kept across sets.  AF: float4 chunks of each of a thread's rows of
+// A read ahead during an exchange, as many as the registers hold beside P.
+template <int KB, int CS, int NTC, int RPT, int AF>
+__device__ __forceinline__ bool cluster_solve_set(const MatrixF32& M, const int* __restrict__ S,
                                                   int k, long long set, const SetOutputs& out,
                                                   ClusterSmem<KB, CS, NTC>& sm,
-                                                  cg::cluster_group& cl, int rank) {
+                                                  cg::cluster_group& cl, int rank, uint32_t& ph) {
   using C = CfgC<KB, CS, NTC, RPT>;
   constexpr int R = C::R, RS = C::RS, TPR = C::TPR, CPT = C::CPT, NCH = C::NCH;
+  constexpr int NPART = ClusterSmem<KB, CS, NTC>::NPART;
+  constexpr int RPW = 32 / TPR;        // row slots per warp
   const int t = threadIdx.x;
-  const int ls = t / TPR;              // row slot: local rows ls + q * RS
+  const int ls = (t >> 5) * RPW + t % RPW;  // row slot: local rows ls + q * RS
   int r[RPT];                          // global rows
 #pragma unroll
   for (int q = 0; q < RPT; ++q) r[q] = rank * R + ls + q * RS;
-  const int g0 = t % TPR;              // owned chunks g0 + TPR * ch
-  const bool lead = g0 == 0;
-  const unsigned rmask = (TPR == 32) ? 0xffffffffu : (((1u << TPR) - 1u) << ((t & 31) / TPR * TPR));
+  const int g0 = (t & 31) / RPW;       // owned chunks g0 + TPR * ch
+  const int w_id = t >> 5, lane = t & 31;
+  // the row whose sums this lane ends with, and the peers it sends them to
+  const int ro = rank * R + ls + g0 / C::CPR * RS;
+  const bool lead = g0 % C::CPR == 0;  // one lane per row contributes to the scalars
+  const uint32_t ybar = smem_u32(&sm.bar[0]), wbar = smem_u32(&sm.bar[1]);
+  // One exchange: the lane's row sum x into row ro of dst in every CTA, then
+  // the warp's partial into part[slot].  (Peer addresses are formed here: held
+  // across the step they would not fit the registers.)
+  auto publish_row = [&](float* dst, float x, uint32_t bar) {
+    if constexpr (CS == 1) {
+      if (lead) dst[ro] = x;
+    } else {
+      const uint32_t a = smem_u32(dst + ro);
+#pragma unroll
+      for (int i = 0; i < C::NP; ++i) {
+        const int p = g0 % C::CPR + i * C::CPR;
+        if (CS % C::CPR == 0 || p < CS) st_async(peer_addr(a, p), x, peer_addr(bar, p));
+      }
+    }
+  };
+  auto publish_partial = [&](int slot, double x, uint32_t bar) {
+    double* pd = &sm.part[slot][rank * C::NWC + w_id];
+    if constexpr (CS == 1) {
+      if (lane == 0) *pd = x;
+    } else {
+      if (lane < CS) st_async(peer_addr(smem_u32(pd), lane), x, peer_addr(bar, lane));
+    }
+  };
+  bool ok = true;
+  auto arrived = [&](uint32_t bar) {
+    if constexpr (CS == 1) {
+      __syncthreads();
+    } else {
+      if (ok) ok = mbar_wait(bar, ph, (volatile int*)&sm.abort, nullptr);
+    }
+  };
 
   // ---- indices (every CTA keeps the full set), validation -------------------
   const SetMatrix SM = set_matrix(M, set);
@@ -139,7 +243,7 @@ __device__ __forceinline__ void cluster_solve_set(const MatrixF32& M, const int*
   if (badsum != 0.0) {
     if (rank == 0 && t == 0) write_failed(out, set, 0, 0, SET_BAD_INDEX);
     set_sync<CS>(cl);
-    return;
+    return true;
   }
 
   // ---- gather own rows of A_S into shared memory; P = I ----------------------
@@ -154,11 +258,12 @@ __device__ __forceinline__ void cluster_solve_set(const MatrixF32& M, const int*
     constexpr int NP = KB / 2, TPP = NTC / NP, PER = (KB + TPP) / TPP;
     static_assert(NP * TPP == NTC, "row pairs per CTA");
     float* __restrict__ Af = reinterpret_cast<float*>(sm.A);
-    // float offset of element (row, col): chunk cc = col / 4 of row
-    // q * RS + ls is held by thread ls * TPR + cc % TPR as its chunk (q, cc / TPR)
+    // float offset of element (row, col): chunk cc = col / 4 of row q * RS + ls
+    // is held by the thread of slot ls and g = cc % TPR as its chunk (q, cc / TPR)
     auto at = [](int row, int col) {
-      const int cc = col >> 2;
-      return ((((row / RS) * NCH + cc / TPR) * NTC + (row % RS) * TPR + cc % TPR) << 2) + (col & 3);
+      const int cc = col >> 2, sl = row % RS;
+      const int th = (sl / RPW) * 32 + (cc % TPR) * RPW + sl % RPW;
+      return ((((row / RS) * NCH + cc / TPR) * NTC + th) << 2) + (col & 3);
     };
     const int p = t % NP, i0 = (t / NP) * PER;
     const int r0 = p, r1 = KB - 1 - p;
@@ -214,12 +319,16 @@ __device__ __forceinline__ void cluster_solve_set(const MatrixF32& M, const int*
   const double tau2 = (32.0 * (double)kEps32) * (32.0 * (double)kEps32) * fro2;
 
   // vb[cur] holds the unnormalised v_j (v_j = sc * vb[cur]), vb[prv] v_{j-1}
-  // (scaled by scp); w is published into vb[nxt].  Peers write vb[nxt] and yb
-  // only after a cluster barrier that follows every read of the old contents.
+  // (scaled by scp); w is published into vb[nxt].  No buffer is written while
+  // it may still be read: a CTA sends y of step j + 1 only after every warp of
+  // the set has sent w of step j, hence after its reads of yb and part[0]; it
+  // sends w of step j only after every warp has sent y of step j, hence after
+  // step j - 1's reads of what is now vb[nxt] and of part[1].
   const float v0 = (float)(1.0 / sqrt((double)k));
   float v[RPT];
 #pragma unroll
   for (int q = 0; q < RPT; ++q) v[q] = r[q] < k ? v0 : 0.f;
+  float vo = ro < k ? v0 : 0.f;  // v of row ro
   for (int c = t; c < KB; c += NTC) {
     sm.vb[0][c] = c < k ? v0 : 0.f;
     sm.vb[1][c] = 0.f;
@@ -229,8 +338,21 @@ __device__ __forceinline__ void cluster_solve_set(const MatrixF32& M, const int*
   int status = 0;
   int cur = 0, prv = 1, nxt = 2;
   __syncthreads();
+  // A's first AF chunks of a pass are read ahead, while w travels
+  static_assert(AF >= 0 && AF <= NCH, "chunks read ahead");
+  float4 ah[AF > 0 ? AF : 1][RPT];
+#pragma unroll
+  for (int ch = 0; ch < AF; ++ch)
+#pragma unroll
+    for (int q = 0; q < RPT; ++q) ah[ch][q] = my[(q * NCH + ch) * NTC];
 
   for (int j = 0; j < k; ++j) {
+    if constexpr (CS > 1) {
+      if (t == 0) {
+        mbar_expect(ybar, exchange_bytes<KB, CS, NTC>());
+        mbar_expect(wbar, exchange_bytes<KB, CS, NTC>());
+      }
+    }
     // P -= v v^T and y = A v over the owned row slices
     float2 ya[RPT], yb[RPT], nc[RPT];
 #pragma unroll
@@ -246,7 +368,7 @@ __device__ __forceinline__ void cluster_solve_set(const MatrixF32& M, const int*
       const float2 b01 = make_float2(b4.x, b4.y), b23 = make_float2(b4.z, b4.w);
 #pragma unroll
       for (int q = 0; q < RPT; ++q) {
-        const float4 a4 = my[(q * NCH + ch) * NTC];
+        const float4 a4 = ch < AF ? ah[ch < AF ? ch : 0][q] : my[(q * NCH + ch) * NTC];
         Pr[q][2 * ch] = __ffma2_rn(nc[q], b01, Pr[q][2 * ch]);
         Pr[q][2 * ch + 1] = __ffma2_rn(nc[q], b23, Pr[q][2 * ch + 1]);
         ya[q] = __ffma2_rn(make_float2(a4.x, a4.y), b01, ya[q]);
@@ -254,30 +376,34 @@ __device__ __forceinline__ void cluster_solve_set(const MatrixF32& M, const int*
       }
     }
     float y[RPT];
-    double ap = 0.0;
 #pragma unroll
-    for (int q = 0; q < RPT; ++q) {
-      y[q] = ((ya[q].x + ya[q].y) + (yb[q].x + yb[q].y)) * sc;
+    for (int q = 0; q < RPT; ++q) y[q] = ((ya[q].x + ya[q].y) + (yb[q].x + yb[q].y)) * sc;
+    const float yo = row_reduce<RPT, TPR>(y, g0);
+    publish_row(sm.yb, yo, ybar);
+    publish_partial(0, warp_sum(lead ? (double)vo * (double)yo : 0.0), ybar);
+    // w~ = y - alpha v_j - beta_j v_{j-1}, every element formed locally (what
+    // does not wait for alpha first)
+    constexpr int NE = (KB + NTC - 1) / NTC;
+    float ve[NE], we[NE];
 #pragma unroll
-      for (int o = TPR / 2; o > 0; o >>= 1) y[q] += __shfl_xor_sync(rmask, y[q], o);
-      ap = q == 0 ? (double)v[0] * (double)y[0] : fma((double)v[q], (double)y[q], ap);
+    for (int e = 0; e < NE; ++e) {
+      const int c = t + e * NTC;
+      ve[e] = c < KB ? sc * sm.vb[cur][c] : 0.f;
+      we[e] = c < KB ? scp * sm.vb[prv][c] : 0.f;
     }
-    // publish the owned rows of y with the alpha partial: one cluster barrier
-    if (lead) {
+    arrived(ybar);
 #pragma unroll
-      for (int p = 0; p < CS; ++p) {
-        ClusterSmem<KB, CS, NTC>* peer = cl.map_shared_rank(&sm, (unsigned)p);
-#pragma unroll
-        for (int q = 0; q < RPT; ++q) peer->yb[r[q]] = y[q];
-      }
-    }
-    const double alpha = cluster_sum<KB, CS, NTC>(lead ? ap : 0.0, sm, 0, cl, rank);
+    for (int e = 0; e < NE; ++e) we[e] = fmaf(-bprev, we[e], t + e * NTC < KB ? sm.yb[t + e * NTC] : 0.f);
+    const double alpha = part_sum<NPART>(sm.part[0]);
     const float af = (float)alpha;
-
-    // w~ = y - alpha v_j - beta_j v_{j-1}, every element formed locally
-    for (int c = t; c < KB; c += NTC)
-      sm.wb[c] = fmaf(-af, sc * sm.vb[cur][c], fmaf(-bprev, scp * sm.vb[prv][c], sm.yb[c]));
-    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < NE; ++e)
+      if (t + e * NTC < KB) sm.wb[t + e * NTC] = fmaf(-af, ve[e], we[e]);
+    if constexpr (CS == 1) {
+      __syncthreads();
+    } else {
+      if (__syncthreads_or(!ok)) break;
+    }
 
     // w = P w~ over the owned row slices
     float2 wa[RPT], wc[RPT];
@@ -296,23 +422,22 @@ __device__ __forceinline__ void cluster_solve_set(const MatrixF32& M, const int*
       }
     }
     float w[RPT];
-    double bp = 0.0;
 #pragma unroll
-    for (int q = 0; q < RPT; ++q) {
-      w[q] = (wa[q].x + wa[q].y) + (wc[q].x + wc[q].y);
+    for (int q = 0; q < RPT; ++q) w[q] = (wa[q].x + wa[q].y) + (wc[q].x + wc[q].y);
+    const float wo = row_reduce<RPT, TPR>(w, g0);
+    publish_row(sm.vb[nxt], wo, wbar);
+    publish_partial(1, warp_sum(lead ? (double)wo * (double)wo : 0.0), wbar);
+    // the next pass's first chunks of A while the rows travel
 #pragma unroll
-      for (int o = TPR / 2; o > 0; o >>= 1) w[q] += __shfl_xor_sync(rmask, w[q], o);
-      bp = q == 0 ? (double)w[0] * (double)w[0] : fma((double)w[q], (double)w[q], bp);
-    }
-    if (lead) {
+    for (int ch = 0; ch < AF; ++ch)
 #pragma unroll
-      for (int p = 0; p < CS; ++p) {
-        ClusterSmem<KB, CS, NTC>* peer = cl.map_shared_rank(&sm, (unsigned)p);
+      for (int q = 0; q < RPT; ++q) ah[ch][q] = my[(q * NCH + ch) * NTC];
+    arrived(wbar);
 #pragma unroll
-        for (int q = 0; q < RPT; ++q) peer->vb[nxt][r[q]] = w[q];
-      }
-    }
-    const double b2v = cluster_sum<KB, CS, NTC>(lead ? bp : 0.0, sm, 1, cl, rank);
+    for (int q = 0; q < RPT; ++q) v[q] = sm.vb[nxt][r[q]];
+    // (after a wait that gave up, the next barrier ends the loop)
+    const double b2v = ok ? part_sum<NPART>(sm.part[1]) : 1.0;
+    ph ^= 1u;
     if (t == 0 && rank == 0) {
       sm.ab[j].x = alpha;
       if (j + 1 < k) sm.ab[j + 1].y = b2v;
@@ -327,8 +452,9 @@ __device__ __forceinline__ void cluster_solve_set(const MatrixF32& M, const int*
       scp = sc;
       sc = 1.0f / bf;
       bprev = bf;
+      vo = wo * sc;
 #pragma unroll
-      for (int q = 0; q < RPT; ++q) v[q] = w[q] * sc;
+      for (int q = 0; q < RPT; ++q) v[q] *= sc;
     } else {
       // Breakdown: restart from the column of P with the largest diagonal
       // (cluster-wide argmax, ties to the smaller row), published into vb[nxt].
@@ -390,25 +516,27 @@ __device__ __forceinline__ void cluster_solve_set(const MatrixF32& M, const int*
         }
       }
       set_sync<CS>(cl);
-      float z[RPT];
-      double zp = 0.0;
-#pragma unroll
-      for (int q = 0; q < RPT; ++q) {
-        z[q] = sm.vb[nxt][r[q]];
-        zp = q == 0 ? (double)z[0] * (double)z[0] : fma((double)z[q], (double)z[q], zp);
-      }
-      const double zz = cluster_sum<KB, CS, NTC>(lead ? zp : 0.0, sm, 2, cl, rank);
+      const float zo = sm.vb[nxt][ro];
+      const double zz = cluster_sum<KB, CS, NTC>(lead ? (double)zo * (double)zo : 0.0, sm, 2, cl, rank);
       if (t == 0 && rank == 0) sm.ab[j + 1].y = 0x1p-600;  // decoupled block (see sturm_count)
       scp = sc;
       sc = 1.0f / sqrtf((float)zz);
       bprev = 0.f;
+      vo = zo * sc;
 #pragma unroll
-      for (int q = 0; q < RPT; ++q) v[q] = z[q] * sc;
+      for (int q = 0; q < RPT; ++q) v[q] = sm.vb[nxt][r[q]] * sc;
     }
     const int old_prv = prv;
     prv = cur;
     cur = nxt;
     nxt = old_prv;
+  }
+  if constexpr (CS > 1) {
+    if (__syncthreads_or(!ok)) {
+      if (rank == 0 && t == 0) write_failed(out, set, 0, 0, SET_NONFINITE);
+      set_sync<CS>(cl);  // every peer's waits give up too; none of its copies is in flight
+      return false;
+    }
   }
   set_sync<CS>(cl);  // every rank done with the step loop before T is read
 
@@ -431,11 +559,11 @@ __device__ __forceinline__ void cluster_solve_set(const MatrixF32& M, const int*
         }
         const double pad = 0x1p-51 * fmax(fabs(glo), fabs(ghi)) + 1e-300;
         const double e = multisect_warp(sm.ab, k, glo - pad, ghi + pad, t < 32 ? 1 : k);
-        if ((t & 31) == 0) sm.part[2][t >> 5] = e;
+        if ((t & 31) == 0) sm.ext[t >> 5] = e;
       }
       __syncthreads();
       if (t == 0) {
-        const double lmin = sm.part[2][0], lmax = sm.part[2][1];
+        const double lmin = sm.ext[0], lmax = sm.ext[1];
         if (out.lmin) out.lmin[set] = lmin;
         if (out.lmax) out.lmax[set] = lmax;
         if (out.delta) out.delta[set] = fmax(1.0 - lmin, lmax - 1.0);
@@ -443,7 +571,8 @@ __device__ __forceinline__ void cluster_solve_set(const MatrixF32& M, const int*
       }
     }
   }
-  set_sync<CS>(cl);  // rank 0's reads of T and part[] precede the next set's writes
+  set_sync<CS>(cl);  // rank 0's reads of T precede the next set's writes
+  return true;
 }
 
 }  // namespace pl

@@ -273,7 +273,7 @@ __global__ void __launch_bounds__(256, 1)
 // Large-k batched form on thread-block clusters (pl_cluster.cuh): persistent,
 // one set per cluster of CS CTAs at a time.
 // ---------------------------------------------------------------------------
-template <int KB, int CS, int NTC, int RPT = 1>
+template <int KB, int CS, int NTC, int RPT, int AF>
 __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NTC, 1)
     k_cluster_solve(MatrixF32 M, SetSource src, SetOutputs out) {
   extern __shared__ __align__(16) float dsm[];
@@ -282,6 +282,16 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NTC, 1)
   const int rank = (int)cl.block_rank();
   const long long ncl = gridDim.x / CS;
   const long long cid = blockIdx.x / CS;
+  if constexpr (CS > 1) {
+    if (threadIdx.x == 0) {
+      mbar_init(smem_u32(&sm.bar[0]), 1);
+      mbar_init(smem_u32(&sm.bar[1]), 1);
+      sm.abort = 0;
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    cl.sync();
+  }
+  uint32_t ph = 0;
   const long long nitems = item_count(src);
   const int pbase = src.perm_start ? *src.perm_start : 0;
   for (long long it = cid; it < nitems; it += ncl) {  // the same items on every rank
@@ -292,7 +302,7 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NTC, 1)
       if (rank == 0 && threadIdx.x == 0) write_failed(out, set, off, 0, SET_BAD_K);
       continue;
     }
-    cluster_solve_set<KB, CS, NTC, RPT>(M, src.idx + off, k, set, out, sm, cl, rank);
+    if (!cluster_solve_set<KB, CS, NTC, RPT, AF>(M, src.idx + off, k, set, out, sm, cl, rank, ph)) return;
   }
 }
 
