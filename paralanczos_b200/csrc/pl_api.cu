@@ -166,12 +166,12 @@ size_t scratch_sar() {
   return grid * (CTA / NT) * (NT / 2) * KB * sizeof(double2);
 }
 
-// shared-A with the next set's triangle prefetched (extremes mode); AR float4
-// chunks of each row of A_S in registers
-template <int KB, int RPT, int CTA, int REGS, int AR = 0>
+// shared-A with the next set's triangle prefetched (extremes mode); NB > 0: A_S
+// in tensor memory
+template <int KB, int RPT, int CTA, int REGS, int NB = 0>
 cudaError_t launch_sap(const MatrixF32& M, const SetSource& src, const SetOutputs& out, long long nitems,
                        void* scratch, cudaStream_t st, bool prep) {
-  auto kern = k_sa_solve_p<KB, RPT, CTA, REGS, AR>;
+  auto kern = k_sa_solve_p<KB, RPT, CTA, REGS, NB>;
   constexpr int GPC = CTA / CfgSA<KB, RPT>::NT;
   const size_t dsm = (sizeof(SASmem<KB, RPT>) + sizeof(SAStage<KB, CfgSA<KB, RPT>::NT>)) * GPC;
   static int occ = [&] {
@@ -188,9 +188,9 @@ cudaError_t launch_sap(const MatrixF32& M, const SetSource& src, const SetOutput
   return cudaGetLastError();
 }
 
-template <int KB, int RPT, int CTA, int REGS, int AR = 0>
+template <int KB, int RPT, int CTA, int REGS, int NB = 0>
 size_t scratch_sap() {
-  auto kern = k_sa_solve_p<KB, RPT, CTA, REGS, AR>;
+  auto kern = k_sa_solve_p<KB, RPT, CTA, REGS, NB>;
   constexpr int NT = CfgSA<KB, RPT>::NT;
   const size_t dsm = (sizeof(SASmem<KB, RPT>) + sizeof(SAStage<KB, CfgSA<KB, RPT>::NT>)) * (CTA / NT);
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm);
@@ -199,12 +199,12 @@ size_t scratch_sap() {
   return grid * (CTA / NT) * (NT / 2) * KB * sizeof(double2);
 }
 
-template <int KB, int CTA, int MINB>
+template <int KB, int CTA, int MINB, int RPT, int NB>
 cudaError_t launch_sa2(const MatrixF32& M, const SetSource& src, const SetOutputs& out,
                        long long nitems, void* scratch, cudaStream_t st, bool prep) {
-  auto kern = k_sa2_solve<KB, CTA, MINB>;
-  constexpr int GPC = CTA / CfgSA2<KB>::NT;
-  const size_t dsm = sizeof(SA2Smem<KB>) * GPC;
+  auto kern = k_sa2_solve<KB, CTA, MINB, RPT, NB>;
+  constexpr int GPC = CTA / CfgSA2<KB, RPT>::NT;
+  const size_t dsm = sizeof(SA2Smem<KB, RPT>) * GPC;
   static int occ = [&] {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm);
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
@@ -219,11 +219,11 @@ cudaError_t launch_sa2(const MatrixF32& M, const SetSource& src, const SetOutput
   return cudaGetLastError();
 }
 
-template <int KB, int CTA, int MINB>
+template <int KB, int CTA, int MINB, int RPT, int NB>
 size_t scratch_sa2() {
-  auto kern = k_sa2_solve<KB, CTA, MINB>;
-  constexpr int NT = CfgSA2<KB>::NT;
-  const size_t dsm = sizeof(SA2Smem<KB>) * (CTA / NT);
+  auto kern = k_sa2_solve<KB, CTA, MINB, RPT, NB>;
+  constexpr int NT = CfgSA2<KB, RPT>::NT;
+  const size_t dsm = sizeof(SA2Smem<KB, RPT>) * (CTA / NT);
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm);
   cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   const size_t grid = (size_t)device_sms() * occupancy(kern, CTA, dsm);
@@ -266,10 +266,10 @@ cudaError_t launch_large(const MatrixF32& M, const SetSource& src, const SetOutp
   return cudaGetLastError();
 }
 
-template <int KB, int CS, int NTC, int RPT = 1, int AF = 0>
+template <int KB, int CS, int NTC, int RPT = 1, int NB = 4>
 cudaError_t launch_cluster(const MatrixF32& M, const SetSource& src, const SetOutputs& out,
                            long long nitems, void*, cudaStream_t st, bool prep) {
-  auto kern = k_cluster_solve<KB, CS, NTC, RPT, AF>;
+  auto kern = k_cluster_solve<KB, CS, NTC, RPT, NB>;
   const size_t dsm = sizeof(ClusterSmem<KB, CS, NTC>);
   static int maxcl = [&] {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm);
@@ -360,28 +360,31 @@ struct Variant {
         {launch_sap<KB, RPT, CTA, REGS>, nullptr}, {scratch_sap<KB, RPT, CTA, REGS>, scratch_none}, \
         true                                                                                     \
   }
-#define SAPR(KB, RPT, CTA, REGS, AR)                                                         \
+// the same with A_S in tensor memory (NB float4 per load)
+#define SAPT(KB, RPT, CTA, REGS, NB)                                                         \
   Variant {                                                                                    \
-    "sharedA prefetch KB=" #KB " RPT=" #RPT " CTA=" #CTA " REGS=" #REGS " AREG=" #AR,          \
-        {launch_sap<KB, RPT, CTA, REGS, AR>, nullptr},                                          \
-        {scratch_sap<KB, RPT, CTA, REGS, AR>, scratch_none}, true                               \
+    "tmemA ahead KB=" #KB " RPT=" #RPT " CTA=" #CTA " REGS=" #REGS " NB=" #NB,                 \
+        {launch_sap<KB, RPT, CTA, REGS, NB>, nullptr},                                          \
+        {scratch_sap<KB, RPT, CTA, REGS, NB>, scratch_none}, true                               \
   }
-#define SA2(KB, CTA, MINB)                                                                   \
+// two threads per row, RPT rows per thread; A_S in tensor memory (NB float4 per load)
+#define SA2(KB, CTA, MINB, RPT, NB)                                                          \
   Variant {                                                                                    \
-    "sharedA 2 threads/row KB=" #KB " CTA=" #CTA " MINB=" #MINB,                               \
-        {launch_sa2<KB, CTA, MINB>, nullptr}, {scratch_sa2<KB, CTA, MINB>, scratch_none}       \
+    "sharedA 2 threads/row KB=" #KB " CTA=" #CTA " MINB=" #MINB " RPT=" #RPT " NB=" #NB,       \
+        {launch_sa2<KB, CTA, MINB, RPT, NB>, nullptr},                                          \
+        {scratch_sa2<KB, CTA, MINB, RPT, NB>, scratch_none}                                     \
   }
 #define CLUSTER(KB, CS, NTC)                                                                  \
   Variant {                                                                                     \
     "cluster KB=" #KB " CS=" #CS " NTC=" #NTC,                                                  \
         {launch_cluster<KB, CS, NTC>, nullptr}, {scratch_none, scratch_none}                    \
   }
-// RPT rows per thread (each with KB / TPR columns of P), AF chunks of A's rows
-// read ahead per step
-#define CLUSTERR(KB, CS, NTC, RPT, AF)                                                            \
+// RPT rows per thread (each with KB / TPR columns of P), A_S read from tensor
+// memory NB float4 at a time
+#define CLUSTERR(KB, CS, NTC, RPT, NB)                                                            \
   Variant {                                                                                     \
     "cluster KB=" #KB " CS=" #CS " NTC=" #NTC " RPT=" #RPT,                                     \
-        {launch_cluster<KB, CS, NTC, RPT, AF>, nullptr}, {scratch_none, scratch_none}           \
+        {launch_cluster<KB, CS, NTC, RPT, NB>, nullptr}, {scratch_none, scratch_none}           \
   }
 // upper 32 x 32 tiles of A_S and P, one set per CTA (NB blocks of 32, NW warps of TPW tiles)
 #define SYM(NB, NW, TPW, MINB)                                                                 \
@@ -406,27 +409,27 @@ const std::vector<Variant>& variants(int b) {
       {SA(48, 3, 128, 2), REG(48, 3, 2, 128, 2)},
       {REG(64, 1, 1, 128, 3), SA(64, 2, 128, 3), REG(64, 1, 1, 128, 2), SA(64, 2, 128, 2),
        SAR(64, 2, 96, 224), SAR(64, 2, 128, 224), SAR(64, 2, 64, 200), SAP(64, 2, 128, 224),
-       SAP(64, 2, 64, 224), SAP(64, 2, 96, 224), SAPR(64, 2, 128, 255, 4), SAPR(64, 2, 64, 255, 4)},
-      {SA(96, 1, 96, 3), SA2(96, 96, 3), SA2(96, 96, 4), SA(96, 1, 96, 4)},
-      {SA(128, 1, 128, 3), REG(128, 1, 2, 256, 1), SA(128, 1, 128, 2), SA2(128, 128, 2), SYM(4, 5, 2, 3),
+       SAP(64, 2, 64, 224), SAP(64, 2, 96, 224), SAPT(64, 2, 256, 224, 4)},
+      {SA(96, 1, 96, 3), SA2(96, 256, 1, 3, 4), SA(96, 1, 96, 4)},
+      {SA(128, 1, 128, 3), REG(128, 1, 2, 256, 1), SA(128, 1, 128, 2), SA2(128, 256, 1, 2, 4), SYM(4, 5, 2, 3),
        SYM(4, 10, 1, 2)},
       {CLUSTER(192, 2, 384), LARGE(256), CLUSTER(192, 4, 192), CLUSTER(192, 1, 384), CLUSTER(192, 1, 768),
-       CLUSTERR(192, 1, 384, 2, 0), CLUSTERR(192, 1, 384, 4, 0), SYM(6, 11, 2, 1), SYM(6, 21, 1, 1),
+       CLUSTERR(192, 1, 384, 2, 4), CLUSTERR(192, 1, 384, 4, 4), SYM(6, 11, 2, 1), SYM(6, 21, 1, 1),
        SYM(6, 16, 2, 1)},
       {CLUSTER(256, 2, 512), LARGE(256), CLUSTER(256, 4, 256), CLUSTER(256, 8, 256), CLUSTER(256, 2, 256),
-       CLUSTERR(256, 2, 256, 2, 0), CLUSTERR(256, 2, 256, 4, 0), SYM(8, 12, 3, 1)},
-      {CLUSTER(384, 4, 384), LARGE(512), CLUSTER(384, 8, 192), CLUSTER(384, 6, 256), CLUSTERR(384, 6, 256, 2, 0),
-       CLUSTERR(384, 6, 256, 4, 4), CLUSTERR(384, 4, 384, 4, 2)},
-      {CLUSTER(512, 8, 256), LARGE(512), CLUSTER(512, 8, 512), CLUSTERR(512, 8, 256, 2, 5),
-       CLUSTERR(512, 8, 256, 4, 0)},
+       CLUSTERR(256, 2, 256, 2, 4), CLUSTERR(256, 2, 256, 4, 4), SYM(8, 12, 3, 1)},
+      {CLUSTER(384, 4, 384), LARGE(512), CLUSTER(384, 8, 192), CLUSTER(384, 6, 256), CLUSTERR(384, 6, 256, 2, 4),
+       CLUSTERR(384, 6, 256, 4, 4), CLUSTERR(384, 4, 384, 4, 4)},
+      {CLUSTER(512, 8, 256), LARGE(512), CLUSTER(512, 8, 512), CLUSTERR(512, 8, 256, 2, 4),
+       CLUSTERR(512, 8, 256, 4, 4)},
   };
   return v[b];
 }
 
 // Built-in shape per bin: the autotuner's choices on B200 (tuning.json), so a
 // caller that never runs the Python tuner (a C program, MATLAB) gets them too.
-const int kDefaultVariant[kNumBins] = {0, 0, 2, 1, 10, 1, 3, 6, 7, 6, 3};
-int g_variant[kNumBins] = {0, 0, 2, 1, 10, 1, 3, 6, 7, 6, 3};
+const int kDefaultVariant[kNumBins] = {0, 0, 1, 1, 10, 1, 3, 6, 7, 6, 3};
+int g_variant[kNumBins] = {0, 0, 1, 1, 10, 1, 3, 6, 7, 6, 3};
 
 int bin_of_k(int k) {
   for (int b = 0; b < kNumBins; ++b)

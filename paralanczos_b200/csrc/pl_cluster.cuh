@@ -3,8 +3,8 @@
 // For 128 < k <= 512 the per-set state (A_S and the projector P, 2 k^2 floats:
 // 512 KB at k = 256, 2 MB at k = 512) does not fit one SM.  A cluster of CS
 // CTAs (one per SM) holds one set: CTA c owns rows [c R, c R + R), R = KB/CS,
-// with its rows of A_S in shared memory (lane-interleaved float4 layout) and
-// its rows of P in registers.  Same recurrence as pl_engine.cuh (three-term
+// with its rows of A_S in tensor memory (pl_tmem.cuh) and its rows of P in
+// registers.  Same recurrence as pl_engine.cuh (three-term
 // step, w = P w~, P -= v v^T fused with the next matvec, FP32 vectors, FP64
 // alpha/beta).  Per step the CTAs exchange, through distributed shared memory:
 // their FP64 partials of alpha and ||w||^2 (one per warp; every warp adds all
@@ -17,10 +17,11 @@
 // the peers with st.async, whose bytes the receiving CTA's mbarrier counts;
 // a warp sends as soon as its rows are done and waits only for the bytes it
 // needs.  No CTA barrier, no cluster barrier (whose release fence the warps
-// would wait for) and no second pass over the partials.  Measured with a
-// cluster barrier per exchange and then with st.async (B200, sets/s): k = 384
-// (1,000 sets) 2.55e4 -> 3.39e4, k = 512 (600 sets) 8.7e3 -> 1.19e4, and with
-// the same reductions inside one CTA k = 192 (3,000 sets) 3.06e5 -> 3.55e5.
+// would wait for) and no second pass over the partials.  Measured (B200,
+// sets/s) with a cluster barrier per exchange and A_S in shared memory, then
+// with st.async, then with A_S in tensor memory: k = 384 (1,000 sets) 2.55e4,
+// 3.39e4, 3.57e4; k = 512 (600 sets) 8.7e3, 1.19e4, 1.41e4; with one CTA per
+// set k = 192 (3,000 sets) 3.06e5, 3.55e5, 4.51e5.
 //
 // Thread mapping inside a CTA: NTC threads; a thread holds RPT of the CTA's
 // R rows (rows ls, ls + R/RPT, ...), TPR = NTC * RPT / R threads share a row;
@@ -41,6 +42,7 @@
 #include "pl_engine.cuh"
 #include "pl_sturm.cuh"
 #include "pl_sync.cuh"
+#include "pl_tmem.cuh"
 
 namespace pl {
 
@@ -70,7 +72,9 @@ struct CfgC {
 template <int KB, int CS, int NTC>
 struct __align__(16) ClusterSmem {
   static constexpr int NPART = CS * (NTC / 32);  // one partial per warp of the set
-  float4 A[(KB / CS) * KB / 4];  // own rows, [chunk][thread]
+  // [float4 of a thread][thread]: P between the segments of the step loop (and,
+  // before the first, where one CTA mirrors its triangle of A_S)
+  float4 P[(KB / CS) * KB / 4];
   float vb[3][KB];               // unnormalised Lanczos vectors, rotating: current, previous, next
   float yb[KB];                  // broadcast of y = A v
   float wb[KB];                  // w~, formed locally from yb
@@ -87,7 +91,7 @@ struct __align__(16) ClusterSmem {
 // What one exchange delivers into every CTA: KB rows and the warps' partials.
 template <int KB, int CS, int NTC>
 __device__ __forceinline__ constexpr uint32_t exchange_bytes() {
-  return KB * sizeof(float) + ClusterSmem<KB, CS, NTC>::NPART * sizeof(double);
+  return KB * sizeof(float) + CS * (NTC / 32) * sizeof(double);
 }
 
 // Address of this CTA's shared-memory address `a` in CTA `rank` of the cluster.
@@ -172,15 +176,27 @@ __device__ __forceinline__ float row_reduce(float (&y)[RPT], int g0) {
   return y[0];
 }
 
-// Solves one set on the cluster.  false: a bounded wait gave up (the set is
-// reported as failed and the kernel must end).  ph: phase parity of the
-// exchanges, kept across sets.  AF: float4 chunks of each of a thread's rows of
-// A read ahead during an exchange, as many as the registers hold beside P.
-template <int KB, int CS, int NTC, int RPT, int AF>
-__device__ __forceinline__ bool cluster_solve_set(const MatrixF32& M, const int* __restrict__ S,
+enum ClusterResult { CLUSTER_DONE, CLUSTER_RESTARTED, CLUSTER_BROKE, CLUSTER_ABORT };
+
+// Solves one set on the cluster.
+//   DONE       its outputs are written
+//   RESTARTED  the same, and it had a breakdown (RESTART)
+//   BROKE      it had a breakdown, nothing is written (!RESTART)
+//   ABORT      a bounded wait gave up: it is reported as failed, and the kernel
+//              must end
+// RESTART: with the breakdown restart.  P then has to outlive the step loop,
+// which costs the loop 80 to 400 bytes of spills at 168 and 255 registers
+// wherever the restart stands (k = 512 1.04 -> 1.25 ms a set, k = 384 0.86 ->
+// 1.32), so a set is first solved without it, and again with it if it breaks
+// down; the two do the same arithmetic.  ph: phase parity of the exchanges,
+// kept across sets.  ta: the thread's tensor memory, read NB float4 at a
+// time.
+template <int KB, int CS, int NTC, int RPT, int NB, bool RESTART>
+__device__ __forceinline__ ClusterResult cluster_solve_set(const MatrixF32& M, const int* __restrict__ S,
                                                   int k, long long set, const SetOutputs& out,
                                                   ClusterSmem<KB, CS, NTC>& sm,
-                                                  cg::cluster_group& cl, int rank, uint32_t& ph) {
+                                                  cg::cluster_group& cl, int rank, uint32_t& ph,
+                                                  uint32_t ta) {
   using C = CfgC<KB, CS, NTC, RPT>;
   constexpr int R = C::R, RS = C::RS, TPR = C::TPR, CPT = C::CPT, NCH = C::NCH;
   constexpr int NPART = ClusterSmem<KB, CS, NTC>::NPART;
@@ -243,12 +259,22 @@ __device__ __forceinline__ bool cluster_solve_set(const MatrixF32& M, const int*
   if (badsum != 0.0) {
     if (rank == 0 && t == 0) write_failed(out, set, 0, 0, SET_BAD_INDEX);
     set_sync<CS>(cl);
-    return true;
+    return CLUSTER_DONE;
   }
 
-  // ---- gather own rows of A_S into shared memory; P = I ----------------------
-  float4* __restrict__ my = sm.A + t;  // chunk (q, ch) at my[(q * NCH + ch) * NTC]
-  float2 Pr[RPT][CPT / 2];
+  // ---- gather own rows of A_S into tensor memory -----------------------------
+  constexpr int NF = NCH * RPT;  // float4 of a thread, (q, ch) as number ch * RPT + q
+  static_assert(NF % NB == 0 && NF % 4 == 0, "whole buffers");
+  // float offset in sm.P of the CTA's element (row, col): chunk cc = col / 4 of
+  // row q * RS + ls belongs to the thread of slot ls and g = cc % TPR as its
+  // (q, cc / TPR)
+  auto at = [](int row, int col) {
+    const int cc = col >> 2, sl = row % RS;
+    const int th = (sl / RPW) * 32 + (cc % TPR) * RPW + sl % RPW;
+    return (((cc / TPR * RPT + row / RS) * NTC + th) << 2) + (col & 3);
+  };
+  float* __restrict__ Pf = reinterpret_cast<float*>(sm.P);
+  float4* __restrict__ my = sm.P + t;  // number i at my[i * NTC]
   double fro = 0.0;
   if constexpr (CS == 1) {
     // One CTA holds all of A_S, which is symmetric: load only its upper
@@ -257,19 +283,11 @@ __device__ __forceinline__ bool cluster_solve_set(const MatrixF32& M, const int*
     // upper elements, shared by TPP threads.
     constexpr int NP = KB / 2, TPP = NTC / NP, PER = (KB + TPP) / TPP;
     static_assert(NP * TPP == NTC, "row pairs per CTA");
-    float* __restrict__ Af = reinterpret_cast<float*>(sm.A);
-    // float offset of element (row, col): chunk cc = col / 4 of row q * RS + ls
-    // is held by the thread of slot ls and g = cc % TPR as its chunk (q, cc / TPR)
-    auto at = [](int row, int col) {
-      const int cc = col >> 2, sl = row % RS;
-      const int th = (sl / RPW) * 32 + (cc % TPR) * RPW + sl % RPW;
-      return ((((row / RS) * NCH + cc / TPR) * NTC + th) << 2) + (col & 3);
-    };
     const int p = t % NP, i0 = (t / NP) * PER;
     const int r0 = p, r1 = KB - 1 - p;
     const float* __restrict__ row0 = SM.A + (size_t)sm.idx[r0] * (size_t)SM.lda;
     const float* __restrict__ row1 = SM.A + (size_t)sm.idx[r1] * (size_t)SM.lda;
-#pragma unroll 4
+#pragma unroll 16
     for (int ii = 0; ii < PER; ++ii) {
       const int i = i0 + ii;
       if (i > KB) break;
@@ -279,40 +297,44 @@ __device__ __forceinline__ bool cluster_solve_set(const MatrixF32& M, const int*
       const float e = (rr < k && c < k) ? __ldg((first ? row0 : row1) + sm.idx[c]) : 0.f;
       const double e2 = (double)e * (double)e;
       fro += (c == rr) ? e2 : 2.0 * e2;
-      Af[at(rr, c)] = e;
-      if (c != rr) Af[at(c, rr)] = e;
+      Pf[at(rr, c)] = e;
+      if (c != rr) Pf[at(c, rr)] = e;
     }
-#pragma unroll
-    for (int q = 0; q < RPT; ++q) {
-      const bool rv = r[q] < k;
-#pragma unroll
-      for (int ch = 0; ch < NCH; ++ch) {
-        const int c = 4 * (g0 + TPR * ch);
-        Pr[q][2 * ch] = make_float2((rv && c == r[q]) ? 1.f : 0.f, (rv && c + 1 == r[q]) ? 1.f : 0.f);
-        Pr[q][2 * ch + 1] =
-            make_float2((rv && c + 2 == r[q]) ? 1.f : 0.f, (rv && c + 3 == r[q]) ? 1.f : 0.f);
-      }
-    }
+    __syncthreads();
+#pragma unroll 4
+    for (int i = 0; i < NF; ++i) tmem_st4(ta, 4 * i, my[i * NTC]);
   } else {
+    // (a rolled loop: 4 U loads in flight)
+    constexpr int U = NF % 8 ? 4 : 8;
+#pragma unroll 1
+    for (int i0 = 0; i0 < NF; i0 += U) {
+      float e[U][4];
 #pragma unroll
-    for (int q = 0; q < RPT; ++q) {
-      const bool rv = r[q] < k;
-      const float* __restrict__ arow = SM.A + (size_t)sm.idx[r[q]] * (size_t)SM.lda;
+      for (int u = 0; u < U; ++u) {
+        const int q = (i0 + u) % RPT, ch = (i0 + u) / RPT;
+        const int row = rank * R + ls + q * RS;
+        const bool rv = row < k;
+        const float* __restrict__ arow = SM.A + (size_t)sm.idx[row] * (size_t)SM.lda;
 #pragma unroll
-      for (int ch = 0; ch < NCH; ++ch) {
-        float e[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int c = 4 * (g0 + TPR * ch) + u;
-          e[u] = (rv && c < k) ? __ldg(arow + sm.idx[c]) : 0.f;
-          fro += (double)e[u] * (double)e[u];
+        for (int v = 0; v < 4; ++v) {
+          const int c = 4 * (g0 + TPR * ch) + v;
+          e[u][v] = (rv && c < k) ? __ldg(arow + sm.idx[c]) : 0.f;
         }
-        my[(q * NCH + ch) * NTC] = make_float4(e[0], e[1], e[2], e[3]);
-        const int c = 4 * (g0 + TPR * ch);
-        Pr[q][2 * ch] = make_float2((rv && c == r[q]) ? 1.f : 0.f, (rv && c + 1 == r[q]) ? 1.f : 0.f);
-        Pr[q][2 * ch + 1] =
-            make_float2((rv && c + 2 == r[q]) ? 1.f : 0.f, (rv && c + 3 == r[q]) ? 1.f : 0.f);
       }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+#pragma unroll
+        for (int v = 0; v < 4; ++v) fro += (double)e[u][v] * (double)e[u][v];
+        tmem_st4(ta, 4 * (i0 + u), make_float4(e[u][0], e[u][1], e[u][2], e[u][3]));
+      }
+    }
+  }
+  tmem_st_wait();
+  if constexpr (RESTART) {  // P = I
+    for (int i = 0; i < NF; ++i) {
+      const int row = rank * R + ls + (i % RPT) * RS, c = 4 * (g0 + TPR * (i / RPT));
+      const bool rv = row < k;
+      my[i * NTC] = make_float4(rv && c == row, rv && c + 1 == row, rv && c + 2 == row, rv && c + 3 == row);
     }
   }
   const double fro2 = cluster_sum<KB, CS, NTC>(fro, sm, 2, cl, rank);
@@ -338,15 +360,28 @@ __device__ __forceinline__ bool cluster_solve_set(const MatrixF32& M, const int*
   int status = 0;
   int cur = 0, prv = 1, nxt = 2;
   __syncthreads();
-  // A's first AF chunks of a pass are read ahead, while w travels
-  static_assert(AF >= 0 && AF <= NCH, "chunks read ahead");
-  float4 ah[AF > 0 ? AF : 1][RPT];
+  // Steps run in segments: a breakdown leaves the step loop, restarts the
+  // recurrence from P in shared memory and enters the loop again.
+  TmemBuf<NB> buf[2];
+  for (int j = 0;; ++j) {
+    float2 Pr[RPT][CPT / 2];
 #pragma unroll
-  for (int ch = 0; ch < AF; ++ch)
+    for (int q = 0; q < RPT; ++q)
 #pragma unroll
-    for (int q = 0; q < RPT; ++q) ah[ch][q] = my[(q * NCH + ch) * NTC];
-
-  for (int j = 0; j < k; ++j) {
+      for (int ch = 0; ch < NCH; ++ch) {
+        if constexpr (RESTART) {
+          const float2* p2 = reinterpret_cast<const float2*>(my + (ch * RPT + q) * NTC);
+          Pr[q][2 * ch] = p2[0];
+          Pr[q][2 * ch + 1] = p2[1];
+        } else {  // I
+          const int c = 4 * (g0 + TPR * ch);
+          const bool rv = r[q] < k;
+          Pr[q][2 * ch] = make_float2(rv && c == r[q], rv && c + 1 == r[q]);
+          Pr[q][2 * ch + 1] = make_float2(rv && c + 2 == r[q], rv && c + 3 == r[q]);
+        }
+      }
+    buf[0].load(ta, 0);
+    for (;; ++j) {
     if constexpr (CS > 1) {
       if (t == 0) {
         mbar_expect(ybar, exchange_bytes<KB, CS, NTC>());
@@ -368,7 +403,12 @@ __device__ __forceinline__ bool cluster_solve_set(const MatrixF32& M, const int*
       const float2 b01 = make_float2(b4.x, b4.y), b23 = make_float2(b4.z, b4.w);
 #pragma unroll
       for (int q = 0; q < RPT; ++q) {
-        const float4 a4 = ch < AF ? ah[ch < AF ? ch : 0][q] : my[(q * NCH + ch) * NTC];
+        const int i = ch * RPT + q, bi = i / NB;
+        if (i % NB == 0) {
+          buf[bi & 1].ready();
+          if ((bi + 1) * NB < NF) buf[(bi + 1) & 1].load(ta, 4 * NB * (bi + 1));
+        }
+        const float4 a4 = buf[bi & 1].f4(i % NB);
         Pr[q][2 * ch] = __ffma2_rn(nc[q], b01, Pr[q][2 * ch]);
         Pr[q][2 * ch + 1] = __ffma2_rn(nc[q], b23, Pr[q][2 * ch + 1]);
         ya[q] = __ffma2_rn(make_float2(a4.x, a4.y), b01, ya[q]);
@@ -402,7 +442,7 @@ __device__ __forceinline__ bool cluster_solve_set(const MatrixF32& M, const int*
     if constexpr (CS == 1) {
       __syncthreads();
     } else {
-      if (__syncthreads_or(!ok)) break;
+      if (__syncthreads_or(!ok)) goto done;
     }
 
     // w = P w~ over the owned row slices
@@ -427,11 +467,7 @@ __device__ __forceinline__ bool cluster_solve_set(const MatrixF32& M, const int*
     const float wo = row_reduce<RPT, TPR>(w, g0);
     publish_row(sm.vb[nxt], wo, wbar);
     publish_partial(1, warp_sum(lead ? (double)wo * (double)wo : 0.0), wbar);
-    // the next pass's first chunks of A while the rows travel
-#pragma unroll
-    for (int ch = 0; ch < AF; ++ch)
-#pragma unroll
-      for (int q = 0; q < RPT; ++q) ah[ch][q] = my[(q * NCH + ch) * NTC];
+    buf[0].load(ta, 0);  // the next pass's first buffer
     arrived(wbar);
 #pragma unroll
     for (int q = 0; q < RPT; ++q) v[q] = sm.vb[nxt][r[q]];
@@ -444,98 +480,91 @@ __device__ __forceinline__ bool cluster_solve_set(const MatrixF32& M, const int*
     }
     if (!isfinite(alpha) || !isfinite(b2v)) {
       status |= SET_NONFINITE;
-      break;
+      goto done;
     }
-    if (j + 1 == k) break;
-    if (b2v > tau2) {
-      const float bf = sqrtf((float)b2v);
-      scp = sc;
-      sc = 1.0f / bf;
-      bprev = bf;
-      vo = wo * sc;
+    if (j + 1 == k) goto done;
+    if (!(b2v > tau2)) break;
+    const float bf = sqrtf((float)b2v);
+    scp = sc;
+    sc = 1.0f / bf;
+    bprev = bf;
+    vo = wo * sc;
 #pragma unroll
-      for (int q = 0; q < RPT; ++q) v[q] *= sc;
-    } else {
-      // Breakdown: restart from the column of P with the largest diagonal
-      // (cluster-wide argmax, ties to the smaller row), published into vb[nxt].
-      status |= SET_BREAKDOWN;
-      unsigned long long kk = 0ull;
-#pragma unroll
-      for (int q = 0; q < RPT; ++q) {
-        if (r[q] < k && (r[q] >> 2) % TPR == g0) {  // this thread owns column r[q] of row r[q]
-          float d = 0.f;
-#pragma unroll
-          for (int ch = 0; ch < NCH; ++ch) {
-            const int c = 4 * (g0 + TPR * ch);
-            if (c == r[q]) d = Pr[q][2 * ch].x;
-            if (c + 1 == r[q]) d = Pr[q][2 * ch].y;
-            if (c + 2 == r[q]) d = Pr[q][2 * ch + 1].x;
-            if (c + 3 == r[q]) d = Pr[q][2 * ch + 1].y;
-          }
-          d = fmaxf(d, 0.f);
-          const unsigned long long kq =
-              ((unsigned long long)__float_as_uint(d) << 32) | (unsigned)(0x7fffffff - r[q]);
-          kk = kq > kk ? kq : kk;
-        }
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long y2 = __shfl_xor_sync(0xffffffffu, kk, o);
-        kk = y2 > kk ? y2 : kk;
-      }
-      if ((t & 31) == 0) sm.red[t >> 5] = __longlong_as_double((long long)kk);
-      __syncthreads();
-      if (t < CS) {
-        unsigned long long m = 0;
-        for (int i = 0; i < NTC / 32; ++i) {
-          const unsigned long long y2 = (unsigned long long)__double_as_longlong(sm.red[i]);
-          m = y2 > m ? y2 : m;
-        }
-        cl.map_shared_rank(&sm, (unsigned)t)->key[rank] = m;
-      }
-      set_sync<CS>(cl);
-      unsigned long long best = 0;
-#pragma unroll
-      for (int q = 0; q < CS; ++q) best = sm.key[q] > best ? sm.key[q] : best;
-      const int mrow = 0x7fffffff - (int)(best & 0xffffffffu);
-#pragma unroll
-      for (int q = 0; q < RPT; ++q) {
-        if (r[q] == mrow) {
-#pragma unroll
-          for (int p = 0; p < CS; ++p) {
-            float* dst = cl.map_shared_rank(&sm, (unsigned)p)->vb[nxt];
-#pragma unroll
-            for (int ch = 0; ch < NCH; ++ch) {
-              const int c = 4 * (g0 + TPR * ch);
-              dst[c] = Pr[q][2 * ch].x;
-              dst[c + 1] = Pr[q][2 * ch].y;
-              dst[c + 2] = Pr[q][2 * ch + 1].x;
-              dst[c + 3] = Pr[q][2 * ch + 1].y;
-            }
-          }
-        }
-      }
-      set_sync<CS>(cl);
-      const float zo = sm.vb[nxt][ro];
-      const double zz = cluster_sum<KB, CS, NTC>(lead ? (double)zo * (double)zo : 0.0, sm, 2, cl, rank);
-      if (t == 0 && rank == 0) sm.ab[j + 1].y = 0x1p-600;  // decoupled block (see sturm_count)
-      scp = sc;
-      sc = 1.0f / sqrtf((float)zz);
-      bprev = 0.f;
-      vo = zo * sc;
-#pragma unroll
-      for (int q = 0; q < RPT; ++q) v[q] = sm.vb[nxt][r[q]] * sc;
-    }
+    for (int q = 0; q < RPT; ++q) v[q] *= sc;
     const int old_prv = prv;
     prv = cur;
     cur = nxt;
     nxt = old_prv;
   }
+    buf[0].ready();  // no load outlives the segment
+    if constexpr (!RESTART) return CLUSTER_BROKE;
+    // Breakdown: restart from the column of P with the largest diagonal
+    // (cluster-wide argmax, ties to the smaller row), published into vb[nxt].
+    status |= SET_BREAKDOWN;
+#pragma unroll
+    for (int q = 0; q < RPT; ++q)
+#pragma unroll
+      for (int ch = 0; ch < NCH; ++ch) {
+        float2* p2 = reinterpret_cast<float2*>(my + (ch * RPT + q) * NTC);
+        p2[0] = Pr[q][2 * ch];
+        p2[1] = Pr[q][2 * ch + 1];
+      }
+    __syncthreads();
+    unsigned long long kk = 0ull;
+    for (int e = t; e < R && rank * R + e < k; e += NTC) {
+      const int row = rank * R + e;
+      const float d = fmaxf(Pf[at(e, row)], 0.f);
+      const unsigned long long kq = ((unsigned long long)__float_as_uint(d) << 32) | (unsigned)(0x7fffffff - row);
+      kk = kq > kk ? kq : kk;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long y2 = __shfl_xor_sync(0xffffffffu, kk, o);
+      kk = y2 > kk ? y2 : kk;
+    }
+    if ((t & 31) == 0) sm.red[t >> 5] = __longlong_as_double((long long)kk);
+    __syncthreads();
+    if (t < CS) {
+      unsigned long long m = 0;
+      for (int i = 0; i < NTC / 32; ++i) {
+        const unsigned long long y2 = (unsigned long long)__double_as_longlong(sm.red[i]);
+        m = y2 > m ? y2 : m;
+      }
+      cl.map_shared_rank(&sm, (unsigned)t)->key[rank] = m;
+    }
+    set_sync<CS>(cl);
+    unsigned long long best = 0;
+#pragma unroll
+    for (int q = 0; q < CS; ++q) best = sm.key[q] > best ? sm.key[q] : best;
+    const int mrow = 0x7fffffff - (int)(best & 0xffffffffu);
+    if (mrow / R == rank) {
+      for (int e = t; e < CS * KB; e += NTC) {
+        ClusterSmem<KB, CS, NTC>* peer = CS == 1 ? &sm : cl.map_shared_rank(&sm, (unsigned)(e / KB));
+        peer->vb[nxt][e % KB] = Pf[at(mrow - rank * R, e % KB)];
+      }
+    }
+    set_sync<CS>(cl);
+    const float zo = sm.vb[nxt][ro];
+    const double zz = cluster_sum<KB, CS, NTC>(lead ? (double)zo * (double)zo : 0.0, sm, 2, cl, rank);
+    if (t == 0 && rank == 0) sm.ab[j + 1].y = 0x1p-600;  // decoupled block (see sturm_count)
+    scp = sc;
+    sc = 1.0f / sqrtf((float)zz);
+    bprev = 0.f;
+    vo = zo * sc;
+#pragma unroll
+    for (int q = 0; q < RPT; ++q) v[q] = sm.vb[nxt][r[q]] * sc;
+    const int old_prv = prv;
+    prv = cur;
+    cur = nxt;
+    nxt = old_prv;
+  }
+done:
+  buf[0].ready();  // no load outlives the set
   if constexpr (CS > 1) {
     if (__syncthreads_or(!ok)) {
       if (rank == 0 && t == 0) write_failed(out, set, 0, 0, SET_NONFINITE);
       set_sync<CS>(cl);  // every peer's waits give up too; none of its copies is in flight
-      return false;
+      return CLUSTER_ABORT;
     }
   }
   set_sync<CS>(cl);  // every rank done with the step loop before T is read
@@ -572,7 +601,7 @@ __device__ __forceinline__ bool cluster_solve_set(const MatrixF32& M, const int*
     }
   }
   set_sync<CS>(cl);  // rank 0's reads of T precede the next set's writes
-  return true;
+  return (status & SET_BREAKDOWN) ? CLUSTER_RESTARTED : CLUSTER_DONE;
 }
 
 }  // namespace pl

@@ -88,22 +88,28 @@ __device__ __forceinline__ Grp<NT> make_group() {
 // (B200, dependent chain), and no shuffles through the shared-memory pipe.
 // All 32 lanes must call it.
 __device__ __forceinline__ double warp_sum(double x) {
-  double c0, c1, d0, d1;
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%4,%4};"
-               : "=d"(c0), "=d"(c1)
-               : "d"(1.0), "d"(x), "d"(0.0));
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%4,%4};"
-               : "=d"(d0), "=d"(d1)
-               : "d"(1.0), "d"(c0 + c1), "d"(0.0));
-  return d0;
+  double s;
+  asm volatile(
+      "{\n\t.reg .f64 one, zero, c0, c1, d1;\n\t"
+      "mov.f64 one, 0d3FF0000000000000;\n\t"
+      "mov.f64 zero, 0d0000000000000000;\n\t"
+      "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {c0, c1}, {one}, {%1}, {zero, zero};\n\t"
+      "add.rn.f64 c0, c0, c1;\n\t"
+      "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, d1}, {one}, {c0}, {zero, zero};\n\t}"
+      : "=d"(s)
+      : "d"(x));
+  return s;
 }
 
 // Sum over the group; identical (bitwise) result in every thread.
 template <int NT, int NW>
 __device__ __forceinline__ double group_sum(double x, const Grp<NT>& g, double* red) {
-  constexpr int W = NT < 32 ? NT : 32;
+  if constexpr (NT < 32) {
 #pragma unroll
-  for (int o = W / 2; o > 0; o >>= 1) x += __shfl_xor_sync(g.mask, x, o);
+    for (int o = NT / 2; o > 0; o >>= 1) x += __shfl_xor_sync(g.mask, x, o);
+  } else {
+    x = warp_sum(x);
+  }
   if constexpr (NW == 1) {
     return x;
   } else {

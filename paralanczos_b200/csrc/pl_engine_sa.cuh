@@ -9,12 +9,19 @@
 // warp shuffles) and twice as many sets are in flight per SM, which is what
 // the latency-bound per-step chain y -> alpha -> w~ -> P w~ -> beta needs.
 //
+// With NB > 0 A_S goes on from shared memory into tensor memory (pl_tmem.cuh)
+// once per set and is streamed from there: the shared-memory pipe, at 59 % with
+// A_S in it, is the busiest unit.  Measured at k = 64 (B200, 200,000 sets): 11.7
+// M sets/s; with the FP64 sums on the matrix unit (warp_sum) 13.4 M; with A_S
+// in tensor memory 14.5 M.
+//
 // A layout: thread t of a group of NT owns rows r_q = t + q*NT (q < RPT); its
 // row data is stored lane-interleaved, A[q][chunk][t][4] (4 floats per chunk),
 // so every thread's LDS.128 of its own row chunk is conflict-free and uses a
 // compile-time offset from one per-thread base pointer.
 #pragma once
 #include "pl_engine.cuh"
+#include "pl_tmem.cuh"
 
 namespace pl {
 
@@ -130,13 +137,13 @@ struct TriPrefetch {
   }
 };
 
-template <int KB, int RPT, bool ALL, bool PF = false, int AR = 0>
+template <int KB, int RPT, bool ALL, bool PF = false, int NB = 0>
 __device__ __forceinline__ int solve_set_sa(const MatrixF32& M, const int* __restrict__ S, int k,
                                              long long set, long long off, const SetOutputs& out,
                                              SASmem<KB, RPT>& sm,
                                              const Grp<CfgSA<KB, RPT>::NT>& g,
                                              SAStage<KB, KB / RPT>* stg = nullptr, bool have = false,
-                                             const SANext* nx = nullptr, bool* issued = nullptr) {
+                                             const SANext* nx = nullptr, bool* issued = nullptr, uint32_t ta = 0) {
   using C = CfgSA<KB, RPT>;
   constexpr int NT = C::NT;
   constexpr int NW = C::NW;
@@ -283,15 +290,17 @@ __device__ __forceinline__ int solve_set_sa(const MatrixF32& M, const int* __res
   float sc = 1.f, bprev = 0.f;
   int status = 0;
   g.sync();
-  // The first AR float4 chunks of each of the thread's rows of A_S are held in
-  // registers for the whole recurrence: AR * RPT fewer shared-memory loads per
-  // step (the L1 data pipe is the kernel's busiest unit), same products.
-  static_assert(AR >= 0 && AR <= NCH, "register chunks of a row");
-  float4 Ar[RPT][AR > 0 ? AR : 1];
+  // the thread's rows of A_S into tensor memory, and the first buffer of the
+  // first pass
+  constexpr int NF = NCH * RPT;
+  static_assert(NB == 0 || (NT == 32 && NF % (NB ? NB : 1) == 0), "one warp per set, whole buffers");
+  [[maybe_unused]] TmemBuf<NB ? NB : 4> buf[2];
+  if constexpr (NB > 0) {
 #pragma unroll
-  for (int q = 0; q < RPT; ++q)
-#pragma unroll
-    for (int ch = 0; ch < AR; ++ch) Ar[q][ch] = my[(q * NCH + ch) * NT];
+    for (int i = 0; i < NF; ++i) tmem_st4(ta, 4 * i, my[((i % RPT) * NCH + i / RPT) * NT]);
+    tmem_st_wait();
+    buf[0].load(ta, 0);
+  }
 
   for (int j = 0; j < k; ++j) {
     if constexpr (PF) pre.step(stg, t);
@@ -310,7 +319,17 @@ __device__ __forceinline__ int solve_set_sa(const MatrixF32& M, const int* __res
       const float2 b01 = make_float2(b4.x, b4.y), b23 = make_float2(b4.z, b4.w);
 #pragma unroll
       for (int q = 0; q < RPT; ++q) {
-        const float4 a4 = ch < AR ? Ar[q][ch < AR ? ch : 0] : my[(q * NCH + ch) * NT];
+        float4 a4;
+        if constexpr (NB > 0) {
+          const int i = ch * RPT + q, bi = i / NB;
+          if (i % NB == 0) {
+            buf[bi & 1].ready();
+            if ((bi + 1) * NB < NF) buf[(bi + 1) & 1].load(ta, 4 * NB * (bi + 1));
+          }
+          a4 = buf[bi & 1].f4(i % NB);
+        } else {
+          a4 = my[(q * NCH + ch) * NT];
+        }
         Pr[q][2 * ch] = __ffma2_rn(ncoef[q], b01, Pr[q][2 * ch]);
         Pr[q][2 * ch + 1] = __ffma2_rn(ncoef[q], b23, Pr[q][2 * ch + 1]);
         ya[q] = __ffma2_rn(make_float2(a4.x, a4.y), b01, ya[q]);
@@ -360,6 +379,7 @@ __device__ __forceinline__ int solve_set_sa(const MatrixF32& M, const int* __res
       bp = fma((double)ww[q], (double)ww[q], bp);
       sm.vb[t + q * NT] = ww[q];  // published by the sync below
     }
+    if constexpr (NB > 0) buf[0].load(ta, 0);  // the next pass's first buffer
     const double b2v = group_sum<NT, NW>(bp, g, sm.red[1]);
     if constexpr (NW == 1) g.sync();
     if (t == 0) {
@@ -430,6 +450,7 @@ __device__ __forceinline__ int solve_set_sa(const MatrixF32& M, const int* __res
       for (int q = 0; q < RPT; ++q) v[q] = z[q] * inv;
     }
   }
+  if constexpr (NB > 0) buf[0].ready();  // no load outlives the set
   g.sync();  // T visible to every thread
   if constexpr (PF) {
     pre.finish(stg, t);  // what the steps left (small k, early exit)

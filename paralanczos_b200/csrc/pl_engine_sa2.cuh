@@ -2,60 +2,72 @@
 //
 // The recurrence of pl_engine_sa.cuh (three-term step, w = P w~ with the
 // explicit projector, P -= v v^T fused with the next matvec; FP32 vectors,
-// FP64 alpha/beta), for 64 < k <= 128 with a group of NT = 128 threads (four
-// warps) per set laid out differently: each thread holds RPT = 2 rows and, of
-// each, every TPR = 2nd float4 column chunk (columns 4 (h + 2 ch) .. +3,
-// h = t % 2).  The projector takes the same 128 registers per thread as with
-// one full row per thread, but every thread reads only its half of the
-// broadcast vectors v and w~, so a warp's broadcast loads per step halve
-// (the shared-memory loads of the one-row-per-thread shape are two thirds
-// A_S, one third broadcasts).  Row sums are finished with one xor-shuffle
-// between the two threads of a row.  Extremes only (the all-eigenvalue mode
-// uses the other shapes of the bin).
+// FP64 alpha/beta), for 64 < k <= 128: each thread of a set's group holds RPT
+// rows and, of each, every TPR = 2nd float4 column chunk (columns
+// 4 (h + 2 ch) .. +3, h = t % 2).  The projector takes KB^2 / NT registers per
+// thread (128 at k <= 128 with RPT = 2 and four warps per set, 144 at k <= 96
+// with RPT = 3 and two), and a thread reads only its half of the broadcast
+// vectors v and w~, once for all of its rows.  Row sums are finished with one
+// xor-shuffle between the two threads of a row.  Extremes only (the
+// all-eigenvalue mode uses the other shapes of the bin).
 //
-// A layout: element (r, c), r = rs + q * NR, chunk cc = c / 4 = h + 2 ch,
-// lives at float4 index (q * NCHT + ch) * NT + (rs * 2 + h): a thread's chunks
-// are conflict-free LDS.128 at compile-time offsets from one base pointer.
+// A_S goes through shared memory once per set, where the gather mirrors its
+// triangle, and from there into tensor memory (pl_tmem.cuh), which every step
+// streams while the shared-memory pipe carries only the broadcasts and the
+// sums.  Measured (B200, 50,000 sets of a 4096-column matrix, sets/s): k = 96
+// 2.99e6 with A_S in shared memory and three warps per set, 3.87e6; k = 128
+// 1.36e6, 1.74e6 (of the latter's gain a third is the FP64 sums on the matrix
+// unit, warp_sum).
+//
+// Layout of A_S in shared memory: element (r, c), r = rs + q * NR, chunk
+// cc = c / 4 = h + 2 ch, lives at float4 index (q * NCHT + ch) * NT + (rs * 2 + h):
+// a thread's chunks are conflict-free LDS.128 at compile-time offsets from one
+// base pointer.
 #pragma once
 #include "pl_engine_sa.cuh"
+#include "pl_tmem.cuh"
 
 namespace pl {
 
-template <int KB>
+// Greatest common divisor (thread shares of a triangle).
+__host__ __device__ constexpr int gcd(int a, int b) { return b == 0 ? a : gcd(b, a % b); }
+
+template <int KB, int RPT_ = 2>
 struct CfgSA2 {
-  static constexpr int RPT = 2, TPR = 2;
+  static constexpr int RPT = RPT_, TPR = 2;
   static constexpr int NR = KB / RPT;        // row slots
   static constexpr int NT = NR * TPR;        // threads per set
   static constexpr int NCHT = KB / 4 / TPR;  // float4 chunks per thread and row
   static constexpr int NW = NT / 32;
-  static_assert(NT % 32 == 0 && KB % (4 * TPR) == 0, "bad shape");
+  static_assert(KB % RPT == 0 && NT % 32 == 0 && KB % (4 * TPR) == 0, "bad shape");
 };
 
-template <int KB>
+template <int KB, int RPT>
 struct __align__(16) SA2Smem {
   float4 A[KB * KB / 4];
   float vb[KB];
   float wb[KB];
   int idx[KB];
   double2 ab[KB];
-  double red[6][CfgSA2<KB>::NW];
+  double red[6][CfgSA2<KB, RPT>::NW];
 };
 
-template <int KB>
+template <int KB, int RPT>
 __device__ __forceinline__ int sa2_at(int r, int c) {
-  using C = CfgSA2<KB>;
+  using C = CfgSA2<KB, RPT>;
   const int q = r / C::NR, rs = r % C::NR, cc = c >> 2;
   return (((q * C::NCHT + cc / C::TPR) * C::NT + rs * C::TPR + cc % C::TPR) << 2) + (c & 3);
 }
 
 // One set on the group (extremes mode: T is left in sm.ab).  Returns the
 // status bits, or -1 if the set failed (its outputs are written).
-template <int KB>
+template <int KB, int RPT, int NB>
 __device__ __forceinline__ int solve_set_sa2(const MatrixF32& M, const int* __restrict__ S, int k,
                                               long long set, long long off, const SetOutputs& out,
-                                              SA2Smem<KB>& sm, const Grp<CfgSA2<KB>::NT>& g) {
-  using C = CfgSA2<KB>;
-  constexpr int NT = C::NT, NW = C::NW, NR = C::NR, RPT = C::RPT, TPR = C::TPR, NCHT = C::NCHT;
+                                              SA2Smem<KB, RPT>& sm, const Grp<CfgSA2<KB, RPT>::NT>& g,
+                                              uint32_t ta = 0) {
+  using C = CfgSA2<KB, RPT>;
+  constexpr int NT = C::NT, NW = C::NW, NR = C::NR, TPR = C::TPR, NCHT = C::NCHT;
   const int t = g.t;
   const int rs = t / TPR, h = t % TPR;
   const bool lead = h == 0;  // the thread of a row that contributes its row to sums
@@ -101,25 +113,27 @@ __device__ __forceinline__ int solve_set_sa2(const MatrixF32& M, const int* __re
     // the upper triangle only (k(k+1)/2 random elements, each its own L1
     // request), each off-diagonal element stored twice; rows p and KB-1-p
     // form a pair of KB+1 upper elements shared by TPP threads
-    constexpr int NP = KB / 2, TPP = NT / NP, PER = (KB + TPP) / TPP;
-    static_assert(NP * TPP == NT, "row pairs per group");
+    // (the least TPP for which the threads take whole shares)
+    constexpr int NP = KB / 2, TPP = NT / gcd(NP, NT), PER = (KB + TPP) / TPP;
     float* __restrict__ Af = reinterpret_cast<float*>(sm.A);
-    const int p = t % NP, i0 = (t / NP) * PER;
-    const int r0 = p, r1 = KB - 1 - p;
-    const float* __restrict__ row0 = SM.A + (size_t)sm.idx[r0] * (size_t)SM.lda;
-    const float* __restrict__ row1 = SM.A + (size_t)sm.idx[r1] * (size_t)SM.lda;
-#pragma unroll 8
-    for (int ii = 0; ii < PER; ++ii) {
-      const int i = i0 + ii;
-      if (TPP > 1 && i > KB) break;
-      const bool first = i < KB - p;
-      const int r = first ? r0 : r1;
-      const int c = first ? p + i : i - 1;  // c >= r
-      const float e = (r < k && c < k) ? __ldg((first ? row0 : row1) + sm.idx[c]) : 0.f;
-      const double e2 = (double)e * (double)e;
-      fro += (c == r) ? e2 : 2.0 * e2;
-      Af[sa2_at<KB>(r, c)] = e;
-      if (c != r) Af[sa2_at<KB>(c, r)] = e;
+    for (int s = t; s < NP * TPP; s += NT) {
+      const int p = s % NP, i0 = (s / NP) * PER;
+      const int r0 = p, r1 = KB - 1 - p;
+      const float* __restrict__ row0 = SM.A + (size_t)sm.idx[r0] * (size_t)SM.lda;
+      const float* __restrict__ row1 = SM.A + (size_t)sm.idx[r1] * (size_t)SM.lda;
+#pragma unroll 16
+      for (int ii = 0; ii < PER; ++ii) {
+        const int i = i0 + ii;
+        if (TPP > 1 && i > KB) break;
+        const bool first = i < KB - p;
+        const int r = first ? r0 : r1;
+        const int c = first ? p + i : i - 1;  // c >= r
+        const float e = (r < k && c < k) ? __ldg((first ? row0 : row1) + sm.idx[c]) : 0.f;
+        const double e2 = (double)e * (double)e;
+        fro += (c == r) ? e2 : 2.0 * e2;
+        Af[sa2_at<KB, RPT>(r, c)] = e;
+        if (c != r) Af[sa2_at<KB, RPT>(c, r)] = e;
+      }
     }
   }
   float2 Pr[RPT][NCHT * 2];  // P's column pairs of the owned chunks
@@ -151,6 +165,17 @@ __device__ __forceinline__ int solve_set_sa2(const MatrixF32& M, const int* __re
   float sc = 1.f, bprev = 0.f;
   int status = 0;
   g.sync();
+  // the thread's row parts of A_S into tensor memory, and the first buffer of
+  // the first pass
+  constexpr int NF = NCHT * RPT;
+  static_assert(NB == 0 || NF % (NB ? NB : 1) == 0, "whole buffers");
+  [[maybe_unused]] TmemBuf<NB ? NB : 4> buf[2];
+  if constexpr (NB > 0) {
+#pragma unroll
+    for (int i = 0; i < NF; ++i) tmem_st4(ta, 4 * i, my[((i % RPT) * NCHT + i / RPT) * NT]);
+    tmem_st_wait();
+    buf[0].load(ta, 0);
+  }
 
   for (int j = 0; j < k; ++j) {
     // P -= v v^T and y = A v over the owned chunks
@@ -168,7 +193,17 @@ __device__ __forceinline__ int solve_set_sa2(const MatrixF32& M, const int* __re
       const float2 b01 = make_float2(b4.x, b4.y), b23 = make_float2(b4.z, b4.w);
 #pragma unroll
       for (int q = 0; q < RPT; ++q) {
-        const float4 a4 = my[(q * NCHT + ch) * NT];
+        float4 a4;
+        if constexpr (NB > 0) {
+          const int i = ch * RPT + q, bi = i / NB;
+          if (i % NB == 0) {
+            buf[bi & 1].ready();
+            if ((bi + 1) * NB < NF) buf[(bi + 1) & 1].load(ta, 4 * NB * (bi + 1));
+          }
+          a4 = buf[bi & 1].f4(i % NB);
+        } else {
+          a4 = my[(q * NCHT + ch) * NT];
+        }
         Pr[q][2 * ch] = __ffma2_rn(ncoef[q], b01, Pr[q][2 * ch]);
         Pr[q][2 * ch + 1] = __ffma2_rn(ncoef[q], b23, Pr[q][2 * ch + 1]);
         ya[q] = __ffma2_rn(make_float2(a4.x, a4.y), b01, ya[q]);
@@ -224,6 +259,7 @@ __device__ __forceinline__ int solve_set_sa2(const MatrixF32& M, const int* __re
         sm.vb[rs + q * NR] = ww[q];  // published by the barrier inside group_sum
       }
     }
+    if constexpr (NB > 0) buf[0].load(ta, 0);  // the next pass's first buffer
     const double b2v = group_sum<NT, NW>(bp, g, sm.red[1]);
     if (t == 0) {
       sm.ab[j].x = alpha;
@@ -302,6 +338,7 @@ __device__ __forceinline__ int solve_set_sa2(const MatrixF32& M, const int* __re
       for (int q = 0; q < RPT; ++q) v[q] = z[q] * inv;
     }
   }
+  if constexpr (NB > 0) buf[0].ready();  // no load outlives the set
   g.sync();  // T visible to every thread
   return status;
 }

@@ -52,14 +52,6 @@ struct __align__(16) SymSmem {
   int idx[KB];
 };
 
-// Sum over the warp; every lane gets the bitwise-same value (xor butterfly of
-// commutative adds).
-__device__ __forceinline__ double sym_warp_sum(double x) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-  return x;
-}
-
 // Sum of N partials in index order (every caller gets the bitwise-same value).
 template <int N>
 __device__ __forceinline__ double sym_sum(const double* p) {
@@ -235,7 +227,7 @@ __device__ __forceinline__ void sym_solve_set(const MatrixF32& M, const int* __r
       }
     }
   }
-  fro = sym_warp_sum(fro);
+  fro = warp_sum(fro);
   if (lane == 0) sm.pb[w] = fro;
   const float v0 = (float)(1.0 / sqrt((double)k));
   for (int c = t; c < KB; c += NTH) {
@@ -302,7 +294,7 @@ __device__ __forceinline__ void sym_solve_set(const MatrixF32& M, const int* __r
       sm.ys[I][J][lane] = sc * sym_rows(rs, cg);
       if (!diag) sm.ys[J][I][8 * cg + rg] = sc * sym_cols(cs, rg);
     }
-    ap = sym_warp_sum(ap) * ((double)sc * (double)sc);
+    ap = warp_sum(ap) * ((double)sc * (double)sc);
     if (lane == 0) sm.pa[w] = ap;
     __syncthreads();
 
@@ -331,7 +323,7 @@ __device__ __forceinline__ void sym_solve_set(const MatrixF32& M, const int* __r
       if (I < nb)
         for (int J = 0; J < nb; ++J) wv += sm.ys[I][J][lane];
       sm.wb[nxt][t] = wv;
-      const double bp = sym_warp_sum((double)wv * (double)wv);
+      const double bp = warp_sum((double)wv * (double)wv);
       if (lane == 0) sm.pb[w] = bp;
     }
     __syncthreads();
@@ -391,7 +383,7 @@ __device__ __forceinline__ void sym_solve_set(const MatrixF32& M, const int* __r
         if (I < nb)
           for (int J = 0; J < nb; ++J) z += sm.ys[I][J][lane];
         sm.wb[nxt][t] = z;
-        const double zp = sym_warp_sum((double)z * (double)z);
+        const double zp = warp_sum((double)z * (double)z);
         if (lane == 0) sm.pz[w] = zp;
       }
       __syncthreads();

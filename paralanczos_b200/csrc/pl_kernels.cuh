@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(CTA, MINB)
 // Batched form, shared-A engine (pl_engine_sa.cuh): persistent, A_S in
 // dynamic shared memory, P in registers.
 // ---------------------------------------------------------------------------
-template <int KB, int RPT, int CTA, bool ALL, bool PF = false, int AR = 0>
+template <int KB, int RPT, int CTA, bool ALL, bool PF = false, int NB = 0>
 __device__ __forceinline__ void sa_solve_body(const MatrixF32& M, const SetSource& src, const SetOutputs& out,
                                               double2* __restrict__ qbuf) {
   using C = CfgSA<KB, RPT>;
@@ -92,6 +92,8 @@ __device__ __forceinline__ void sa_solve_body(const MatrixF32& M, const SetSourc
   // after the GPC SASmem slots)
   SAStage<KB, C::NT>* stg = PF ? reinterpret_cast<SAStage<KB, C::NT>*>(smem + GPC) + gic : nullptr;
   bool have = false;  // stg holds this set's elements
+  TmemA<4 * C::NCH * RPT, CTA, NB> am;
+  am.begin();
   int nq = 0;
   for (long long it = (long long)blockIdx.x * GPC + gic; it < nitems; it += ng) {
     long long set, off;
@@ -120,8 +122,8 @@ __device__ __forceinline__ void sa_solve_body(const MatrixF32& M, const SetSourc
       if (g.t == 0) qmeta[gic][nq] = QueueMeta{set, k, 0};
     }
     bool issued = false;
-    const int st = solve_set_sa<KB, RPT, ALL, PF, AR>(M, src.idx + off, k, set, off, out, smem[gic], g, stg, have,
-                                                  &nx, &issued);
+    const int st = solve_set_sa<KB, RPT, ALL, PF, NB>(M, src.idx + off, k, set, off, out, smem[gic], g, stg, have,
+                                                  &nx, &issued, am.ta);
     have = issued;
     if constexpr (!ALL) {
       if (st >= 0) {
@@ -142,6 +144,7 @@ __device__ __forceinline__ void sa_solve_body(const MatrixF32& M, const SetSourc
     if (nq > 0) queue_bisect(T, Q, nq, qmeta[gic], g.t, out, g.mask);
   }
   if constexpr (PF) cp_async_wait_all();  // no copy outlives the kernel
+  am.end();
 }
 
 template <int KB, int RPT, int CTA, int MINB, bool ALL>
@@ -159,27 +162,29 @@ __global__ void __maxnreg__(REGS) k_sa_solve_r(MatrixF32 M, SetSource src, SetOu
 }
 
 // The same with the next set's triangle prefetched into a shared-memory stage
-// (extremes mode); AR float4 chunks of each row of A_S also held in registers.
-template <int KB, int RPT, int CTA, int REGS, int AR = 0>
+// (extremes mode); NB > 0: A_S in tensor memory, read NB float4 at a time.
+template <int KB, int RPT, int CTA, int REGS, int NB = 0>
 __global__ void __maxnreg__(REGS) k_sa_solve_p(MatrixF32 M, SetSource src, SetOutputs out,
                                                double2* __restrict__ qbuf) {
-  sa_solve_body<KB, RPT, CTA, false, true, AR>(M, src, out, qbuf);
+  sa_solve_body<KB, RPT, CTA, false, true, NB>(M, src, out, qbuf);
 }
 
 // ---------------------------------------------------------------------------
 // Batched form, shared-A engine with two threads per row (pl_engine_sa2.cuh),
 // extremes only: persistent, A_S in dynamic shared memory, P in registers.
 // ---------------------------------------------------------------------------
-template <int KB, int CTA, int MINB>
+template <int KB, int CTA, int MINB, int RPT = 2, int NB = 0>
 __global__ void __launch_bounds__(CTA, MINB)
     k_sa2_solve(MatrixF32 M, SetSource src, SetOutputs out, double2* __restrict__ qbuf) {
-  using C = CfgSA2<KB>;
+  using C = CfgSA2<KB, RPT>;
   constexpr int GPC = CTA / C::NT;
   constexpr int Q = C::NT / 2;
   static_assert(CTA % C::NT == 0 && GPC <= 15, "CTA must hold whole groups");
   extern __shared__ __align__(16) float dsm[];
-  SA2Smem<KB>* smem = reinterpret_cast<SA2Smem<KB>*>(dsm);
+  SA2Smem<KB, RPT>* smem = reinterpret_cast<SA2Smem<KB, RPT>*>(dsm);
   __shared__ QueueMeta qmeta[GPC][Q];
+  TmemA<4 * C::NCHT * RPT, CTA, NB> am;
+  am.begin();
   const Grp<C::NT> g = make_group<C::NT>();
   const int gic = threadIdx.x / C::NT;
   const long long ng = (long long)gridDim.x * GPC;
@@ -196,7 +201,7 @@ __global__ void __launch_bounds__(CTA, MINB)
       continue;
     }
     if (g.t == 0) qmeta[gic][nq] = QueueMeta{set, k, 0};
-    const int st = solve_set_sa2<KB>(M, src.idx + off, k, set, off, out, smem[gic], g);
+    const int st = solve_set_sa2<KB, RPT, NB>(M, src.idx + off, k, set, off, out, smem[gic], g, am.ta);
     if (st >= 0) {
       const int kq = qmeta[gic][nq].k;
       for (int i = g.t; i < kq; i += C::NT) T[(size_t)i * Q + nq] = smem[gic].ab[i];
@@ -211,6 +216,7 @@ __global__ void __launch_bounds__(CTA, MINB)
     }
   }
   if (nq > 0) queue_bisect(T, Q, nq, qmeta[gic], g.t, out, g.mask);
+  am.end();
 }
 
 // ---------------------------------------------------------------------------
@@ -273,7 +279,7 @@ __global__ void __launch_bounds__(256, 1)
 // Large-k batched form on thread-block clusters (pl_cluster.cuh): persistent,
 // one set per cluster of CS CTAs at a time.
 // ---------------------------------------------------------------------------
-template <int KB, int CS, int NTC, int RPT, int AF>
+template <int KB, int CS, int NTC, int RPT, int NB>
 __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NTC, 1)
     k_cluster_solve(MatrixF32 M, SetSource src, SetOutputs out) {
   extern __shared__ __align__(16) float dsm[];
@@ -292,6 +298,10 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NTC, 1)
     cl.sync();
   }
   uint32_t ph = 0;
+  TmemA<KB / CS * KB / NTC, NTC, NB> am;
+  am.begin();
+  ClusterResult res = CLUSTER_DONE;
+  bool likely_breaks = false;
   const long long nitems = item_count(src);
   const int pbase = src.perm_start ? *src.perm_start : 0;
   for (long long it = cid; it < nitems; it += ncl) {  // the same items on every rank
@@ -302,8 +312,22 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NTC, 1)
       if (rank == 0 && threadIdx.x == 0) write_failed(out, set, off, 0, SET_BAD_K);
       continue;
     }
-    if (!cluster_solve_set<KB, CS, NTC, RPT, AF>(M, src.idx + off, k, set, out, sm, cl, rank, ph)) return;
+    // one CTA: the loop fits its registers with the restart (0.30 ms a set
+    // either way at k = 192, and a breakdown costs no second solve).  A set after
+    // one that broke down is likely to break down too.
+    if constexpr (CS > 1) {
+      if (!likely_breaks) {
+        res = cluster_solve_set<KB, CS, NTC, RPT, NB, false>(M, src.idx + off, k, set, out, sm, cl, rank, ph, am.ta);
+        likely_breaks = res == CLUSTER_BROKE;
+      }
+    }
+    if (CS == 1 || likely_breaks) {
+      res = cluster_solve_set<KB, CS, NTC, RPT, NB, true>(M, src.idx + off, k, set, out, sm, cl, rank, ph, am.ta);
+      likely_breaks = res == CLUSTER_RESTARTED;
+    }
+    if (res == CLUSTER_ABORT) break;
   }
+  am.end();
 }
 
 // ---------------------------------------------------------------------------
