@@ -70,11 +70,12 @@ int occupancy(K kern, int cta, size_t dsmem) {
   return occ > 0 ? occ : 1;
 }
 
-long long grid_for(long long nitems, int per_cta, int occ) {
+// CTAs of a persistent launch: the full grid, or one per item if that is less
+// (a CTA's groups take items a whole grid apart).
+long long grid_for(long long nitems, int occ) {
   const long long full = (long long)device_sms() * occ;
-  if (nitems < 0) return full;  // count lives on the device
-  const long long need = (nitems + per_cta - 1) / per_cta;
-  return need < full ? (need > 0 ? need : 1) : full;
+  if (nitems < 0 || nitems >= full) return full;  // nitems < 0: the count lives on the device
+  return nitems > 0 ? nitems : 1;
 }
 
 template <int KB, int RPT, int TPR, int CTA, int MINB, bool ALL>
@@ -86,8 +87,7 @@ cudaError_t launch_reg(const MatrixF32& M, const SetSource& src, const SetOutput
     cudaFuncAttributes fa;
     return cudaFuncGetAttributes(&fa, kern);
   }
-  constexpr int GPC = CTA / Cfg<KB, RPT, TPR>::NT;
-  const long long grid = grid_for(nitems, GPC, occ);
+  const long long grid = grid_for(nitems, occ);
   kern<<<(unsigned)grid, CTA, 0, st>>>(M, src, out, (double2*)scratch);
   return cudaGetLastError();
 }
@@ -117,7 +117,7 @@ cudaError_t launch_sa(const MatrixF32& M, const SetSource& src, const SetOutputs
     cudaFuncAttributes fa;
     return cudaFuncGetAttributes(&fa, kern);
   }
-  const long long grid = grid_for(nitems, GPC, occ);
+  const long long grid = grid_for(nitems, occ);
   kern<<<(unsigned)grid, CTA, dsm, st>>>(M, src, out, (double2*)scratch);
   return cudaGetLastError();
 }
@@ -149,7 +149,7 @@ cudaError_t launch_sar(const MatrixF32& M, const SetSource& src, const SetOutput
     cudaFuncAttributes fa;
     return cudaFuncGetAttributes(&fa, kern);
   }
-  const long long grid = grid_for(nitems, GPC, occ);
+  const long long grid = grid_for(nitems, occ);
   kern<<<(unsigned)grid, CTA, dsm, st>>>(M, src, out, (double2*)scratch);
   return cudaGetLastError();
 }
@@ -166,37 +166,41 @@ size_t scratch_sar() {
   return grid * (CTA / NT) * (NT / 2) * KB * sizeof(double2);
 }
 
-// shared-A with the next set's triangle prefetched (extremes mode); NB > 0: A_S
-// in tensor memory
-template <int KB, int RPT, int CTA, int REGS, int NB = 0>
+// shared-A with the next set's triangle prefetched (PF); NB > 0: A_S in tensor
+// memory
+template <int KB, int RPT, int CTA, int REGS, int NB, bool ALL, bool PF>
+struct Sap {
+  static constexpr int NT = CfgSA<KB, RPT>::NT;
+  static constexpr size_t dsm = (sizeof(SASmem<KB, RPT>) + (PF ? sizeof(SAStage<KB, NT>) : 0)) * (CTA / NT);
+  static constexpr auto kern() { return k_sa_solve_p<KB, RPT, CTA, REGS, NB, ALL, PF>; }
+  static int occ() {
+    static int o = [] {
+      cudaFuncSetAttribute(kern(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm);
+      cudaFuncSetAttribute(kern(), cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+      return occupancy(kern(), CTA, dsm);
+    }();
+    return o;
+  }
+};
+
+template <int KB, int RPT, int CTA, int REGS, int NB = 0, bool ALL = false, bool PF = true>
 cudaError_t launch_sap(const MatrixF32& M, const SetSource& src, const SetOutputs& out, long long nitems,
                        void* scratch, cudaStream_t st, bool prep) {
-  auto kern = k_sa_solve_p<KB, RPT, CTA, REGS, NB>;
-  constexpr int GPC = CTA / CfgSA<KB, RPT>::NT;
-  const size_t dsm = (sizeof(SASmem<KB, RPT>) + sizeof(SAStage<KB, CfgSA<KB, RPT>::NT>)) * GPC;
-  static int occ = [&] {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm);
-    cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    return occupancy(kern, CTA, dsm);
-  }();
+  using S = Sap<KB, RPT, CTA, REGS, NB, ALL, PF>;
+  const int occ = S::occ();
   if (prep) {
     cudaFuncAttributes fa;
-    return cudaFuncGetAttributes(&fa, kern);
+    return cudaFuncGetAttributes(&fa, S::kern());
   }
-  const long long grid = grid_for(nitems, GPC, occ);
-  kern<<<(unsigned)grid, CTA, dsm, st>>>(M, src, out, (double2*)scratch);
+  k_sa_solve_p<KB, RPT, CTA, REGS, NB, ALL, PF>
+      <<<(unsigned)grid_for(nitems, occ), CTA, S::dsm, st>>>(M, src, out, (double2*)scratch);
   return cudaGetLastError();
 }
 
 template <int KB, int RPT, int CTA, int REGS, int NB = 0>
 size_t scratch_sap() {
-  auto kern = k_sa_solve_p<KB, RPT, CTA, REGS, NB>;
-  constexpr int NT = CfgSA<KB, RPT>::NT;
-  const size_t dsm = (sizeof(SASmem<KB, RPT>) + sizeof(SAStage<KB, CfgSA<KB, RPT>::NT>)) * (CTA / NT);
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm);
-  cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-  const size_t grid = (size_t)device_sms() * occupancy(kern, CTA, dsm);
-  return grid * (CTA / NT) * (NT / 2) * KB * sizeof(double2);
+  using S = Sap<KB, RPT, CTA, REGS, NB, false, true>;
+  return (size_t)device_sms() * S::occ() * (CTA / S::NT) * (S::NT / 2) * KB * sizeof(double2);
 }
 
 template <int KB, int CTA, int MINB, int RPT, int NB>
@@ -214,7 +218,7 @@ cudaError_t launch_sa2(const MatrixF32& M, const SetSource& src, const SetOutput
     cudaFuncAttributes fa;
     return cudaFuncGetAttributes(&fa, kern);
   }
-  const long long grid = grid_for(nitems, GPC, occ);
+  const long long grid = grid_for(nitems, occ);
   kern<<<(unsigned)grid, CTA, dsm, st>>>(M, src, out, (double2*)scratch);
   return cudaGetLastError();
 }
@@ -261,7 +265,7 @@ cudaError_t launch_large(const MatrixF32& M, const SetSource& src, const SetOutp
     cudaFuncAttributes fa;
     return cudaFuncGetAttributes(&fa, kern);
   }
-  const long long grid = grid_for(nitems, 1, 1);
+  const long long grid = grid_for(nitems, 1);
   kern<<<(unsigned)grid, 256, 0, st>>>(M, src, out, (float*)scratch);
   return cudaGetLastError();
 }
@@ -312,7 +316,7 @@ cudaError_t launch_sym(const MatrixF32& M, const SetSource& src, const SetOutput
     cudaFuncAttributes fa;
     return cudaFuncGetAttributes(&fa, kern);
   }
-  const long long grid = grid_for(nitems, 1, occ);
+  const long long grid = grid_for(nitems, occ);
   if (verbosity() >= 2)
     fprintf(stderr, "paralanczos: sym NB=%d NW=%d TPW=%d: %lld CTAs (%d per SM), %zu B smem/CTA\n", NB, NW, TPW,
             grid, occ, dsm);
@@ -360,18 +364,21 @@ struct Variant {
         {launch_sap<KB, RPT, CTA, REGS>, nullptr}, {scratch_sap<KB, RPT, CTA, REGS>, scratch_none}, \
         true                                                                                     \
   }
-// the same with A_S in tensor memory (NB float4 per load)
+// the same with A_S in tensor memory (NB float4 per load); all eigenvalues at up
+// to 255 registers (the bisection holds 16 rows of T and their minors twice)
 #define SAPT(KB, RPT, CTA, REGS, NB)                                                         \
   Variant {                                                                                    \
     "tmemA ahead KB=" #KB " RPT=" #RPT " CTA=" #CTA " REGS=" #REGS " NB=" #NB,                 \
-        {launch_sap<KB, RPT, CTA, REGS, NB>, nullptr},                                          \
+        {launch_sap<KB, RPT, CTA, REGS, NB>, launch_sap<KB, RPT, CTA, 255, NB, true>},          \
         {scratch_sap<KB, RPT, CTA, REGS, NB>, scratch_none}, true                               \
   }
-// two threads per row, RPT rows per thread; A_S in tensor memory (NB float4 per load)
-#define SA2(KB, CTA, MINB, RPT, NB)                                                          \
+// two threads per row, RPT rows per thread, A_S in tensor memory (NB float4 per
+// load); all eigenvalues: one row per thread (the bin's other FP32 sums) with
+// A_S in tensor memory, ACTA threads of AREGS registers
+#define SA2(KB, CTA, MINB, RPT, NB, ACTA, AREGS)                                             \
   Variant {                                                                                    \
     "sharedA 2 threads/row KB=" #KB " CTA=" #CTA " MINB=" #MINB " RPT=" #RPT " NB=" #NB,       \
-        {launch_sa2<KB, CTA, MINB, RPT, NB>, nullptr},                                          \
+        {launch_sa2<KB, CTA, MINB, RPT, NB>, launch_sap<KB, 1, ACTA, AREGS, NB, true, false>},  \
         {scratch_sa2<KB, CTA, MINB, RPT, NB>, scratch_none}                                     \
   }
 #define CLUSTER(KB, CS, NTC)                                                                  \
@@ -398,6 +405,9 @@ struct Variant {
         {scratch_large<KM>, scratch_large<KM>}                                           \
   }
 
+// most sets per SM of a short call (short_call below)
+constexpr int kShortSetsPerSm = 16;
+
 const int kBinK[] = {8, 16, 32, 48, 64, 96, 128, 192, 256, 384, 512};
 constexpr int kNumBins = 11;
 
@@ -410,8 +420,8 @@ const std::vector<Variant>& variants(int b) {
       {REG(64, 1, 1, 128, 3), SA(64, 2, 128, 3), REG(64, 1, 1, 128, 2), SA(64, 2, 128, 2),
        SAR(64, 2, 96, 224), SAR(64, 2, 128, 224), SAR(64, 2, 64, 200), SAP(64, 2, 128, 224),
        SAP(64, 2, 64, 224), SAP(64, 2, 96, 224), SAPT(64, 2, 256, 224, 4)},
-      {SA(96, 1, 96, 3), SA2(96, 256, 1, 3, 4), SA(96, 1, 96, 4)},
-      {SA(128, 1, 128, 3), REG(128, 1, 2, 256, 1), SA(128, 1, 128, 2), SA2(128, 256, 1, 2, 4), SYM(4, 5, 2, 3),
+      {SA(96, 1, 96, 3), SA2(96, 256, 1, 3, 4, 384, 168), SA(96, 1, 96, 4)},
+      {SA(128, 1, 128, 3), REG(128, 1, 2, 256, 1), SA(128, 1, 128, 2), SA2(128, 256, 1, 2, 4, 256, 255), SYM(4, 5, 2, 3),
        SYM(4, 10, 1, 2)},
       {CLUSTER(192, 2, 384), LARGE(256), CLUSTER(192, 4, 192), CLUSTER(192, 1, 384), CLUSTER(192, 1, 768),
        CLUSTERR(192, 1, 384, 2, 4), CLUSTERR(192, 1, 384, 4, 4), SYM(6, 11, 2, 1), SYM(6, 21, 1, 1),
@@ -546,6 +556,16 @@ bool env_flag(const char* name, bool dflt) {
   return !(v[0] == '0' || v[0] == 'n' || v[0] == 'N' || v[0] == 'f' || v[0] == 'F');
 }
 
+// A short call of 8 < k <= 16 runs on the next bin's kernel, one warp per set
+// instead of a quarter: its sums over a whole warp and its bisection by 16
+// threads per extreme are the shorter dependent chains, and the sets have the
+// SMs to themselves (the FP32 sums are the same: padding adds zeros).
+// 256 sets of k = 16: 30.3 -> 18.6 us on the GPU; equal at 16 sets per SM (28.9),
+// 33 against 41 at 28.
+bool short_call(int b, bool all, long long nsets) {
+  return kBinK[b] == 16 && !all && nsets <= (long long)device_sms() * kShortSetsPerSm;
+}
+
 // Uniform k: one kernel.
 int solve_uniform(const MatrixF32& M, const int* idx, long long nsets, int k, int form,
                   const SetOutputs& out, cudaStream_t st) {
@@ -555,8 +575,9 @@ int solve_uniform(const MatrixF32& M, const int* idx, long long nsets, int k, in
     PL_CU(plain_fn(k, all)(M, src, out, nsets, nullptr, st, false));
     return PL_OK;
   }
-  const int b = bin_of_k(k);
+  int b = bin_of_k(k);
   if (b < 0) return PL_ENOTSUP;
+  if (short_call(b, all, nsets)) ++b;
   const Variant& v = chosen_for(b, all);
   void* scratch = nullptr;
   const size_t need = v.scratch[all ? 1 : 0]();

@@ -147,6 +147,7 @@ __device__ __forceinline__ void cgs_solve_set(const MatrixF32& M, const int* __r
     const double b2v = group_sum<NT, NW>(bp, g, sm.red[1]);
     if (t == 0) {
       sm.ab[j].x = alpha;
+      if (j == 0) sm.ab[0].y = 0.0;
       if (j + 1 < k) sm.ab[j + 1].y = b2v;
     }
     if (!isfinite(alpha) || !isfinite(b2v)) {

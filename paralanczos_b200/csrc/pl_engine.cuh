@@ -242,11 +242,23 @@ __device__ __forceinline__ int solve_set(const MatrixF32& M, const int* __restri
 #pragma unroll
     for (int cc = 0; cc < CPT; cc += 2) {
       const int c = c0 + cc;
-      const float a0 = (rv && c < k) ? __ldg(arow + sm.idx[c]) : 0.f;
-      const float a1 = (rv && c + 1 < k) ? __ldg(arow + sm.idx[c + 1]) : 0.f;
+      const float a0 = (rv & (c < k)) ? __ldg(arow + sm.idx[c]) : 0.f;
+      const float a1 = (rv & (c + 1 < k)) ? __ldg(arow + sm.idx[c + 1]) : 0.f;
       Ar[q][cc / 2] = make_float2(a0, a1);
+    }
+  }
+  // (after all the loads are issued: an FP64 use of each value behind its load
+  // left about one load in flight)
+#pragma unroll
+  for (int q = 0; q < RPT; ++q) {
+    const int r = rowid[q];
+    const bool rv = r < k;
+#pragma unroll
+    for (int cc = 0; cc < CPT; cc += 2) {
+      const int c = c0 + cc;
+      const float2 e = Ar[q][cc / 2];
       Pr[q][cc / 2] = make_float2((rv && c == r) ? 1.f : 0.f, (rv && c + 1 == r) ? 1.f : 0.f);
-      fro += (double)a0 * (double)a0 + (double)a1 * (double)a1;
+      fro += (double)e.x * (double)e.x + (double)e.y * (double)e.y;
     }
   }
   const double fro2 = group_sum<NT, NW>(fro, g, sm.red[2]);
@@ -261,6 +273,7 @@ __device__ __forceinline__ int solve_set(const MatrixF32& M, const int* __restri
     vp[q] = 0.f;
   }
   for (int c = t; c < KB; c += NT) sm.vb[c] = c < k ? v0 : 0.f;
+  if (t == 0) sm.ab[0].y = 0.0;
   float sc = 1.f;     // v = sc * vb (vb holds the unnormalised vector)
   float bprev = 0.f;  // beta_j for the three-term step
   int status = 0;
@@ -434,23 +447,29 @@ __device__ __forceinline__ int solve_set(const MatrixF32& M, const int* __restri
   }
 
   {
-    int R = 0;
-    {
-      double wdt = ghi - glo, tol = bisect_tol(glo, ghi);
-      while (wdt > tol && R < 200) {
-        wdt *= 0.5;
-        ++R;
-      }
-    }
+    const int R = bisect_rounds(glo, ghi);
     double prod = 1.0;
-    for (int m = t; m < k; m += NT) {
-      const double e = bisect_index(sm.ab, k, m, glo, ghi, R);
-      if (out.eig) out.eig[off + m] = e;
-      prod *= e;
-      if (m == 0 && out.lmin) out.lmin[set] = e;
-      if (m == k - 1 && out.lmax) out.lmax[set] = e;
-      if (m == 0) sm.red[4][0] = e;  // lambda_min for delta (read after the sync below)
-      if (m == k - 1) sm.red[5][0] = e;
+    // a thread's eigenvalues two at a time: their chains overlap
+    constexpr int EV = KB > NT ? 2 : 1;
+    for (int m0 = t; m0 < k; m0 += EV * NT) {
+      double lam[EV];
+      bisect_indices<(KB > 32 && KB <= 64 ? 16 : 8), EV>(sm.ab, k, m0, NT, glo, ghi, R, lam);
+#pragma unroll
+      for (int v = 0; v < EV; ++v) {
+        const int m = m0 + v * NT;
+        if (m >= k) break;
+        const double e = lam[v];
+        if (out.eig) out.eig[off + m] = e;
+        prod *= e;
+        if (m == 0) {
+          sm.red[4][0] = e;  // for delta, read after the sync below
+          if (out.lmin) out.lmin[set] = e;
+        }
+        if (m == k - 1) {
+          sm.red[5][0] = e;
+          if (out.lmax) out.lmax[set] = e;
+        }
+      }
     }
     // product over the group (fixed butterfly order, deterministic)
     {

@@ -150,7 +150,7 @@ __device__ __forceinline__ int solve_set_sa(const MatrixF32& M, const int* __res
   constexpr int NCH = C::NCH;
   const int t = g.t;
   if constexpr (PF) {
-    static_assert(RPT <= 2 && !ALL, "the prefetch follows the triangle gather (extremes mode)");
+    static_assert(RPT <= 2, "the prefetch follows the triangle gather");
     *issued = false;
     if (have) cp_async_wait_all();  // this set's stage (issued a whole set ago)
   }
@@ -293,7 +293,7 @@ __device__ __forceinline__ int solve_set_sa(const MatrixF32& M, const int* __res
   // the thread's rows of A_S into tensor memory, and the first buffer of the
   // first pass
   constexpr int NF = NCH * RPT;
-  static_assert(NB == 0 || (NT == 32 && NF % (NB ? NB : 1) == 0), "one warp per set, whole buffers");
+  static_assert(NB == 0 || NF % (NB ? NB : 1) == 0, "whole buffers");
   [[maybe_unused]] TmemBuf<NB ? NB : 4> buf[2];
   if constexpr (NB > 0) {
 #pragma unroll
@@ -482,26 +482,28 @@ __device__ __forceinline__ int solve_set_sa(const MatrixF32& M, const int* __res
     ghi += pad;
   }
   {
-    int R = 0;
-    {
-      double wdt = ghi - glo, tol = bisect_tol(glo, ghi);
-      while (wdt > tol && R < 200) {
-        wdt *= 0.5;
-        ++R;
-      }
-    }
+    const int R = bisect_rounds(glo, ghi);
     double prod = 1.0;
-    for (int m = t; m < k; m += NT) {
-      const double e = bisect_index(sm.ab, k, m, glo, ghi, R);
-      if (out.eig) out.eig[off + m] = e;
-      prod *= e;
-      if (m == 0) {
-        sm.red[4][0] = e;
-        if (out.lmin) out.lmin[set] = e;
-      }
-      if (m == k - 1) {
-        sm.red[5][0] = e;
-        if (out.lmax) out.lmax[set] = e;
+    // a thread's eigenvalues two at a time: their chains overlap
+    constexpr int EV = KB > NT ? 2 : 1;
+    for (int m0 = t; m0 < k; m0 += EV * NT) {
+      double lam[EV];
+      bisect_indices<(KB > 32 && (KB <= 64 || NB > 0) ? 16 : 8), EV>(sm.ab, k, m0, NT, glo, ghi, R, lam);
+#pragma unroll
+      for (int v = 0; v < EV; ++v) {
+        const int m = m0 + v * NT;
+        if (m >= k) break;
+        const double e = lam[v];
+        if (out.eig) out.eig[off + m] = e;
+        prod *= e;
+        if (m == 0) {
+          sm.red[4][0] = e;  // for delta, read after the sync below
+          if (out.lmin) out.lmin[set] = e;
+        }
+        if (m == k - 1) {
+          sm.red[5][0] = e;
+          if (out.lmax) out.lmax[set] = e;
+        }
       }
     }
     constexpr int W = NT < 32 ? NT : 32;

@@ -14,7 +14,10 @@ namespace pl {
 
 // ---------------------------------------------------------------------------
 // Batched form: persistent, register-resident engine for one k bin.
-// Each group of NT threads takes work items gid, gid + ngroups, ...
+// Group g of CTA b takes work items g * gridDim.x + b, + ngroups, ...: fewer
+// items than groups spread over the SMs, one or a few to each, and do not share
+// one SM's gather and shared-memory pipes (256 sets of k = 16: 1,000 instead of
+// 4,100 cycles of gather).
 // ---------------------------------------------------------------------------
 template <int KB, int RPT, int TPR, int CTA, int MINB, bool ALL>
 __global__ void __launch_bounds__(CTA, MINB)
@@ -33,7 +36,7 @@ __global__ void __launch_bounds__(CTA, MINB)
   const int pbase = src.perm_start ? *src.perm_start : 0;
   double2* __restrict__ T = qbuf + ((size_t)blockIdx.x * GPC + gic) * (size_t)(Q * KB);
   int nq = 0;
-  for (long long it = (long long)blockIdx.x * GPC + gic; it < nitems; it += ng) {
+  for (long long it = (long long)gic * gridDim.x + blockIdx.x; it < nitems; it += ng) {
     long long set, off;
     int k;
     set_span(src, it, pbase, set, off, k);
@@ -55,7 +58,7 @@ __global__ void __launch_bounds__(CTA, MINB)
         ++nq;
         g.sync();
         if (nq == Q) {
-          queue_bisect(T, Q, nq, qmeta[gic], g.t, out, g.mask);
+          queue_bisect<KB, C::NT>(T, Q, nq, qmeta[gic], g.t, out, g.mask, nullptr);
           g.sync();
           nq = 0;
         }
@@ -63,7 +66,7 @@ __global__ void __launch_bounds__(CTA, MINB)
     }
   }
   if constexpr (!ALL) {
-    if (nq > 0) queue_bisect(T, Q, nq, qmeta[gic], g.t, out, g.mask);
+    if (nq > 0) queue_bisect<KB, C::NT>(T, Q, nq, qmeta[gic], g.t, out, g.mask, smem[gic].ab);
   }
 }
 
@@ -95,7 +98,7 @@ __device__ __forceinline__ void sa_solve_body(const MatrixF32& M, const SetSourc
   TmemA<4 * C::NCH * RPT, CTA, NB> am;
   am.begin();
   int nq = 0;
-  for (long long it = (long long)blockIdx.x * GPC + gic; it < nitems; it += ng) {
+  for (long long it = (long long)gic * gridDim.x + blockIdx.x; it < nitems; it += ng) {
     long long set, off;
     int k;
     set_span(src, it, pbase, set, off, k);
@@ -133,7 +136,7 @@ __device__ __forceinline__ void sa_solve_body(const MatrixF32& M, const SetSourc
         ++nq;
         g.sync();
         if (nq == Q) {
-          queue_bisect(T, Q, nq, qmeta[gic], g.t, out, g.mask);
+          queue_bisect<KB, C::NT>(T, Q, nq, qmeta[gic], g.t, out, g.mask, nullptr);
           g.sync();
           nq = 0;
         }
@@ -141,7 +144,7 @@ __device__ __forceinline__ void sa_solve_body(const MatrixF32& M, const SetSourc
     }
   }
   if constexpr (!ALL) {
-    if (nq > 0) queue_bisect(T, Q, nq, qmeta[gic], g.t, out, g.mask);
+    if (nq > 0) queue_bisect<KB, C::NT>(T, Q, nq, qmeta[gic], g.t, out, g.mask, smem[gic].ab);
   }
   if constexpr (PF) cp_async_wait_all();  // no copy outlives the kernel
   am.end();
@@ -162,11 +165,11 @@ __global__ void __maxnreg__(REGS) k_sa_solve_r(MatrixF32 M, SetSource src, SetOu
 }
 
 // The same with the next set's triangle prefetched into a shared-memory stage
-// (extremes mode); NB > 0: A_S in tensor memory, read NB float4 at a time.
-template <int KB, int RPT, int CTA, int REGS, int NB = 0>
+// (PF); NB > 0: A_S in tensor memory, read NB float4 at a time.
+template <int KB, int RPT, int CTA, int REGS, int NB, bool ALL, bool PF = true>
 __global__ void __maxnreg__(REGS) k_sa_solve_p(MatrixF32 M, SetSource src, SetOutputs out,
                                                double2* __restrict__ qbuf) {
-  sa_solve_body<KB, RPT, CTA, false, true, NB>(M, src, out, qbuf);
+  sa_solve_body<KB, RPT, CTA, ALL, PF, NB>(M, src, out, qbuf);
 }
 
 // ---------------------------------------------------------------------------
@@ -192,7 +195,7 @@ __global__ void __launch_bounds__(CTA, MINB)
   const int pbase = src.perm_start ? *src.perm_start : 0;
   double2* __restrict__ T = qbuf + ((size_t)blockIdx.x * GPC + gic) * (size_t)(Q * KB);
   int nq = 0;
-  for (long long it = (long long)blockIdx.x * GPC + gic; it < nitems; it += ng) {
+  for (long long it = (long long)gic * gridDim.x + blockIdx.x; it < nitems; it += ng) {
     long long set, off;
     int k;
     set_span(src, it, pbase, set, off, k);
@@ -209,13 +212,13 @@ __global__ void __launch_bounds__(CTA, MINB)
       ++nq;
       g.sync();
       if (nq == Q) {
-        queue_bisect(T, Q, nq, qmeta[gic], g.t, out, g.mask);
+        queue_bisect<KB, C::NT>(T, Q, nq, qmeta[gic], g.t, out, g.mask, nullptr);
         g.sync();
         nq = 0;
       }
     }
   }
-  if (nq > 0) queue_bisect(T, Q, nq, qmeta[gic], g.t, out, g.mask);
+  if (nq > 0) queue_bisect<KB, C::NT>(T, Q, nq, qmeta[gic], g.t, out, g.mask, smem[gic].ab);
   am.end();
 }
 

@@ -3,7 +3,7 @@
 // Replaces the reference's serial one-lane TQLRAT (ParaLanczos.cu:32-189, called
 // at ParaLanczos.cu:1461).  The count of eigenvalues of T below x is the number of
 // sign changes of the leading principal minors of T - xI (continuant form,
-// division-free, with power-of-two rescaling every 8 rows).  The reference's
+// division-free, with power-of-two rescaling every 16 rows).  The reference's
 // own Sturm sketch, EIGVALS_BELOW (ParaLanczos.cu:519-552), is unused and skips
 // alpha[1]; this is new code.  The CPU restatement is orc_sturm_count in
 // oracle/pl_oracle.c.
@@ -12,90 +12,118 @@
 
 namespace pl {
 
-// Power-of-two rescaling of the last two minors, applied when the exponent of
-// p1 leaves [2^-200, 2^200]: exact, keeps signs and ratios.
+// Power-of-two rescaling of the last two minors by p1's exponent: exact, keeps
+// signs and ratios.  (Without a branch: a taken-or-not one costs as much as ten
+// rows.)  A zero p1 leaves them as they are.
 __device__ __forceinline__ void sturm_rescale(double& p0, double& p1) {
-  const int e = ((__double2hiint(p1) >> 20) & 0x7ff) - 1022;  // |p1| = f * 2^e, f in [0.5, 1)
-  if (e > 200 || e < -200) {
-    const int c = e < -1021 ? -1021 : (e > 1021 ? 1021 : e);
-    const double s = __hiloint2double((1023 - c) << 20, 0);  // exactly 2^-c
-    p0 *= s;
-    p1 *= s;
-  }
+  const int f = (__double2hiint(p1) >> 20) & 0x7ff;  // |p1| = m * 2^(f - 1023), m in [1, 2)
+  const int c = f < 2 ? 1023 : (f > 2043 ? 2043 : f);
+  const double s = __hiloint2double((f == 0 ? 1023 : 2046 - c) << 20, 0);  // 2^(1023 - c)
+  p0 *= s;
+  p1 *= s;
 }
 
-// Number of eigenvalues of T strictly below x.  ab[i] = {alpha_i, beta_i^2}
-// (beta_0^2 unused), beta_i^2 > 0 for i >= 1 (a decoupled block stores 2^-600,
-// so two consecutive minors cannot both vanish).  Sign changes of the leading
-// principal minors p_0 = 1, p_i = (alpha_i - x) p_{i-1} - beta_i^2 p_{i-2}; a
-// minor that is exactly zero counts as positive, which gives the right count
-// because its neighbours then have opposite signs.
-__device__ __forceinline__ int sturm_count(const double2* __restrict__ ab, int k, double x) {
-  double p0 = 1.0, p1 = ab[0].x - x;
-  unsigned sp = (unsigned)__double2hiint(p1) >> 31;
-  int cnt = (int)sp;
-  int i = 1;
-  for (; i + 16 <= k; i += 16) {
+// U rows of the minors' recurrence at once: p_i = (alpha_i - x) p_{i-1} -
+// beta_i^2 p_{i-2}.  The signs are looked at only when the U minors are done
+// (the empty asm holds that work behind them): an integer use of a minor right
+// behind it stalls the chain.  Rows r .. U - 1 do not count.
+template <int U>
+__device__ __forceinline__ void sturm_rows(const double2 (&t)[U], int r, double x, double& p0, double& p1,
+                                           unsigned& sp, int& cnt) {
+  static_assert(U == 8 || U == 16, "rows per block");
+  double p[U];
 #pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      const double2 t = ab[i + u];
-      const double p2 = fma(t.x - x, p1, -t.y * p0);
-      const unsigned s2 = (unsigned)__double2hiint(p2) >> 31;
-      cnt += (int)(s2 ^ sp);
-      sp = s2;
-      p0 = p1;
-      p1 = p2;
-    }
-    sturm_rescale(p0, p1);
+  for (int u = 0; u < U; ++u) {
+    const double pm1 = u == 0 ? p1 : p[u > 0 ? u - 1 : 0];
+    const double pm2 = u == 0 ? p0 : (u == 1 ? p1 : p[u > 1 ? u - 2 : 0]);
+    p[u] = fma(t[u].x - x, pm1, -t[u].y * pm2);
   }
-  for (; i < k; ++i) {
-    const double2 t = ab[i];
-    const double p2 = fma(t.x - x, p1, -t.y * p0);
-    const unsigned s2 = (unsigned)__double2hiint(p2) >> 31;
-    cnt += (int)(s2 ^ sp);
-    sp = s2;
-    p0 = p1;
-    p1 = p2;
-  }
-  return cnt;
+  if constexpr (U == 16)
+    asm volatile("" : "+d"(p[8]), "+d"(p[9]), "+d"(p[10]), "+d"(p[11]), "+d"(p[12]), "+d"(p[13]), "+d"(p[14]),
+                      "+d"(p[15]));
+  asm volatile("" : "+d"(p[0]), "+d"(p[1]), "+d"(p[2]), "+d"(p[3]), "+d"(p[4]), "+d"(p[5]), "+d"(p[6]), "+d"(p[7]));
+  unsigned m = sp;  // signs, the newest in bit 0
+#pragma unroll
+  for (int u = 0; u < U; ++u) m = __funnelshift_l((unsigned)__double2hiint(p[u]), m, 1);
+  cnt += __popc((m ^ (m >> 1)) & (((1u << U) - 1u) & ~((1u << (U - r)) - 1u)));
+  sp = m & 1u;
+  p0 = p[U - 2];
+  p1 = p[U - 1];
 }
 
-// Same count over a strided tridiagonal: element i at ab[i * stride].
+// Numbers of eigenvalues of T strictly below x[0 .. E-1].  Element i of T at
+// ab[i * stride] = {alpha_i, beta_i^2}, beta_0^2 = 0, beta_i^2 > 0 for i >= 1 (a
+// decoupled block stores 2^-600, so two consecutive minors cannot both
+// vanish).  Sign changes of the leading principal minors p_{-1} = 0, p_0 = 1,
+// ...; a minor that is exactly zero counts as positive, which gives the right
+// count because its neighbours then have opposite signs.  Rows go in blocks of
+// U, each loaded before its recurrence, the last one filled up with rows that
+// do not count; 25 to 30 cycles a row where loads and signs in the chain took 42
+// (one warp, B200).  E > 1 shares the loads and runs E chains side by side.
+template <int U, int E>
+__device__ __forceinline__ void sturm_counts(const double2* __restrict__ ab, int stride, int k,
+                                             const double (&x)[E], int (&cnt)[E]) {
+  double p0[E], p1[E];
+  unsigned sp[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    p0[e] = 0.0;
+    p1[e] = 1.0;
+    sp[e] = 0u;
+    cnt[e] = 0;
+  }
+  int i = 0;
+  for (; i + U <= k; i += U) {
+    double2 t[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) t[u] = ab[(size_t)(i + u) * stride];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      if (i > 0 && (i & 15) == 0) sturm_rescale(p0[e], p1[e]);
+      sturm_rows<U>(t, U, x[e], p0[e], p1[e], sp[e], cnt[e]);
+    }
+  }
+  if (i < k) {
+    double2 t[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) t[u] = ab[(size_t)(i + u < k ? i + u : k - 1) * stride];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      if (i > 0 && (i & 15) == 0) sturm_rescale(p0[e], p1[e]);
+      sturm_rows<U>(t, k - i, x[e], p0[e], p1[e], sp[e], cnt[e]);
+    }
+  }
+}
+
+template <int U>
 __device__ __forceinline__ int sturm_count_strided(const double2* __restrict__ ab, int stride, int k,
                                                    double x) {
-  double p0 = 1.0, p1 = ab[0].x - x;
-  unsigned sp = (unsigned)__double2hiint(p1) >> 31;
-  int cnt = (int)sp;
-  int i = 1;
-  for (; i + 16 <= k; i += 16) {
-#pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      const double2 t = ab[(size_t)(i + u) * stride];
-      const double p2 = fma(t.x - x, p1, -t.y * p0);
-      const unsigned s2 = (unsigned)__double2hiint(p2) >> 31;
-      cnt += (int)(s2 ^ sp);
-      sp = s2;
-      p0 = p1;
-      p1 = p2;
-    }
-    sturm_rescale(p0, p1);
-  }
-  for (; i < k; ++i) {
-    const double2 t = ab[(size_t)i * stride];
-    const double p2 = fma(t.x - x, p1, -t.y * p0);
-    const unsigned s2 = (unsigned)__double2hiint(p2) >> 31;
-    cnt += (int)(s2 ^ sp);
-    sp = s2;
-    p0 = p1;
-    p1 = p2;
-  }
-  return cnt;
+  const double xs[1] = {x};
+  int cnt[1];
+  sturm_counts<U, 1>(ab, stride, k, xs, cnt);
+  return cnt[0];
+}
+
+__device__ __forceinline__ int sturm_count(const double2* __restrict__ ab, int k, double x) {
+  return sturm_count_strided<8>(ab, 1, k, x);
 }
 
 // Termination width for an interval whose ends have magnitude up to `mag`.
 // 2^-34 (6e-11) of the spectrum's scale: far below the FP32 Lanczos error.
 __device__ __forceinline__ double bisect_tol(double lo, double hi) {
   return 0x1p-34 * fmax(fabs(lo), fabs(hi)) + 1e-300;
+}
+
+// Rounds of bisection needed to shrink [lo, hi] below tol.
+__device__ __forceinline__ int bisect_rounds(double lo, double hi) {
+  double w = hi - lo;
+  const double tol = bisect_tol(lo, hi);
+  int r = 0;
+  while (w > tol && r < 200) {
+    w *= 0.5;
+    ++r;
+  }
+  return r;
 }
 
 // Rounds of (G+1)-way multisection needed to shrink [lo, hi] below tol.
@@ -162,15 +190,38 @@ __device__ __forceinline__ double multisect_warp(const double2* __restrict__ ab,
   return 0.5 * (a + b);
 }
 
-// Eigenvalue number m (0-based, ascending) by R rounds of plain bisection.
+// Eigenvalues number m, m + step, ... (E of them, 0-based, ascending; numbers
+// >= k are left alone) by R rounds of plain bisection, side by side.
+template <int U, int E>
+__device__ __forceinline__ void bisect_indices(const double2* __restrict__ ab, int k, int m, int step,
+                                               double lo, double hi, int R, double (&lam)[E]) {
+  double a[E], b[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    a[e] = lo;
+    b[e] = hi;
+  }
+  for (int r = 0; r < R; ++r) {
+    double x[E];
+    int cnt[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) x[e] = 0.5 * (a[e] + b[e]);
+    sturm_counts<U, E>(ab, 1, k, x, cnt);
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      if (cnt[e] >= m + e * step + 1) b[e] = x[e]; else a[e] = x[e];
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < E; ++e) lam[e] = 0.5 * (a[e] + b[e]);
+}
+
+// Eigenvalue number m.
 __device__ __forceinline__ double bisect_index(const double2* __restrict__ ab, int k, int m,
                                                double lo, double hi, int R) {
-  double a = lo, b = hi;
-  for (int r = 0; r < R; ++r) {
-    const double x = 0.5 * (a + b);
-    if (sturm_count(ab, k, x) >= m + 1) b = x; else a = x;
-  }
-  return 0.5 * (a + b);
+  double lam[1];
+  bisect_indices<8, 1>(ab, k, m, 0, lo, hi, R, lam);
+  return lam[0];
 }
 
 }  // namespace pl
