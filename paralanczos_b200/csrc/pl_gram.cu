@@ -28,7 +28,7 @@
 // of the residual remains.
 //
 // Kernel structure (one persistent CTA per SM, 288 threads):
-//   warps 0-3  gather: cp.async of the set's 128 column records per 64-row
+//   warps 0-3  gather: cp.async of the tile's 128 column records per 64-row
 //              K chunk into a 4-stage ring of SWIZZLE_128B K-major tiles;
 //   warp  8    owns 512 TMEM columns, one elected thread issues tcgen05.mma
 //              and tcgen05.commit;
@@ -202,14 +202,23 @@ __global__ void __launch_bounds__(256) k_gram_colnorm(const float* __restrict__ 
 }
 
 // ---------------------------------------------------------------------------
+// A tile of 128 set positions holds 128 / KP sets of KP = 2^lkp >= k rows each
+// (tile row r: set r / KP, position r % KP); the tensor core forms the whole
+// 128 x 128 product and the epilogue reads each row's own set's columns of it,
+// so a small k costs a fraction of a tile (m = 1024, 20,000 sets of one tile each,
+// then packed: k = 50 1.94 -> 0.93 ms, k = 32 1.88 -> 0.47, k = 16 1.84 -> 0.24).
+//
 // Batched Gram blocks of sets [0, nsets) (uniform k <= 128): block s at
 // blocks + s * k * k, row-major, exactly symmetric.  gerr[s] |= SET_BAD_INDEX
 // for a set with an index outside [0, n) (its rows read as zero).
 // ---------------------------------------------------------------------------
+template <int lkp>
 __global__ void __launch_bounds__(NTHREADS, 1)
     k_gram(const char* __restrict__ prep, const float* __restrict__ nrm2, int n, int kc_total,
            const int* __restrict__ idx, long long nsets, int k, float* __restrict__ blocks,
            int* __restrict__ gerr, int* __restrict__ status, int hold) {
+  constexpr int KP = 1 << lkp, lspt = 7 - lkp;  // rows per set, log2 sets per tile
+  const long long ntiles = (nsets + (1 << lspt) - 1) >> lspt;
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -265,24 +274,27 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     const uint32_t dst0 = (uint32_t)((sg >> 3) * PIECE_BYTES + rsub * 128 + (((sg & 7) ^ rsub) << 4));
     uint32_t it = 0;
     bool ok = true;
-    for (long long set = blockIdx.x; set < nsets && ok; set += gridDim.x) {
+    for (long long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
       const char* src[16];
       uint32_t nbytes = 0;  // 16 if row valid else 0 (zero fill), one bit per row
-      bool bad = false;
+      uint32_t bad = 0;     // rows whose index is outside [0, n)
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
-        const int r = rsub + 8 * i;
+        const int r = rsub + 8 * i, pos = r & (KP - 1);
+        const long long set = (tile << lspt) + (r >> lkp);
         int v = 0;
         bool valid = false;
-        if (r < k) {
-          v = __ldg(idx + set * (long long)k + r);
+        if (pos < k && set < nsets) {
+          v = __ldg(idx + set * (long long)k + pos);
           valid = v >= 0 && v < n;
-          bad |= !valid;
+          bad |= (valid ? 0u : 1u) << i;
         }
         src[i] = prep + (valid ? (size_t)v * rec_stride : 0) + sg * 16;
         nbytes |= (valid ? 1u : 0u) << i;
       }
-      if (bad) atomicOr(gerr + set, SET_BAD_INDEX);
+      // (behind the loop: a store between the index loads would serialise them)
+      for (; bad; bad &= bad - 1)
+        atomicOr(gerr + (tile << lspt) + ((rsub + 8 * (__ffs(bad) - 1)) >> lkp), SET_BAD_INDEX);
       for (int kc = 0; kc < kc_total; ++kc, ++it) {
         const int s = it % NS;
         if (it >= NS && !mbar_wait(empty_bar(s), ((it / NS) - 1) & 1, abort, status)) {
@@ -313,7 +325,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     if ((tid & 31) == 0) {
       uint32_t it = 0, j = 0, G = 0;
       bool ok = !hold;  // hold: issue nothing, so every other role's wait runs out
-      for (long long set = blockIdx.x; set < nsets && ok; set += gridDim.x, ++j) {
+      for (long long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++j) {
         const uint32_t a = j & 1;
         if (j >= 2 && !mbar_wait(d2empty_bar(a), ((j >> 1) - 1) & 1, abort, status)) {
           ok = false;
@@ -367,11 +379,18 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     const int e = tid - NPROD;
     const int q = warp & 3;
     const int row = 32 * q + (tid & 31);
-    const uint32_t lane_base = tmem + ((uint32_t)(32 * q) << 16);
+    // this warp's rows need KE columns from c0 on: their sets' (two sets of 16)
+    constexpr int KE = KP < 32 ? 32 : KP;
+    const int c0 = 32 * q & ~(KE - 1);
+    const int rc = row - c0;                      // the row's own column there
+    const int r0 = row & ~(KP - 1), pos = row - r0;  // first row of its set, its position
+    const uint32_t lane_base = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)c0;
     float* Er = E + row * EPAD;
     uint32_t j = 0, G = 0;
     bool ok = true;
-    for (long long set = blockIdx.x; set < nsets && ok; set += gridDim.x, ++j) {
+    for (long long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++j) {
+      const long long set = (tile << lspt) + (row >> lkp);
+      const bool mine = pos < k && set < nsets;
       const uint32_t a = j & 1;
       // D1 segments: sum into this thread's row of E with round-to-nearest adds
       for (int kc0 = 0; kc0 < kc_total; kc0 += SEG, ++G) {
@@ -384,7 +403,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         }
         tc_fence_after();
 #pragma unroll 1
-        for (int cb = 0; cb < ROWS / 32; ++cb) {
+        for (int cb = 0; cb < KE / 32; ++cb) {
           float u[32];
           tmem_ld32(lane_base + b * 128 + 32 * cb, u);
           tmem_wait_ld();
@@ -406,7 +425,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       if (!*go_d2) break;
       tc_fence_after();
 #pragma unroll 1
-      for (int cb = 0; cb < ROWS / 32; ++cb) {
+      for (int cb = 0; cb < KE / 32; ++cb) {
         float w[32];
         tmem_ld32(lane_base + 256 + a * 128 + 32 * cb, w);
         tmem_wait_ld();
@@ -419,9 +438,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       // diagonal), kept in the row's padding slot of E (column ROWS, never an
       // accumulator); 1 for an invalid index or a non-positive norm
       float dr = 1.f;
-      if (row < k) {
-        const int gi = __ldg(idx + set * (long long)k + row);
-        const float dg = Er[row];
+      if (mine) {
+        const int gi = __ldg(idx + set * (long long)k + pos);
+        const float dg = Er[rc];
         if (gi >= 0 && gi < n) {
           const float ex = __ldg(nrm2 + gi);
           if (ex > 0.f && dg > 0.f) dr = (float)sqrt((double)ex / (double)dg);
@@ -429,13 +448,15 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       }
       Er[ROWS] = dr;
       asm volatile("bar.sync 1, %0;" ::"n"(NEPI) : "memory");
-      if (row < k) {
-        float* dst = blocks + (size_t)set * k * k + row;
-        // (both operand pairs commute, so element (c, row) written by thread
-        // c is bitwise element (row, c): the block stays exactly symmetric)
+      if (mine) {
+        float* dst = blocks + (size_t)set * k * k + pos;
+        const float* Es = E + r0 * EPAD;
+        const float* Ec = Er + (r0 - c0);
+        // (both operand pairs commute, so element (c, pos) written by row pos's
+        // thread is bitwise element (pos, c): the block stays exactly symmetric)
 #pragma unroll 4
         for (int c = 0; c < k; ++c)
-          dst[(size_t)c * k] = (0.5f * (Er[c] + E[c * EPAD + row])) * (dr * E[c * EPAD + ROWS]);
+          dst[(size_t)c * k] = (0.5f * (Ec[c] + Es[c * EPAD + rc])) * (dr * Es[c * EPAD + ROWS]);
       }
       asm volatile("bar.sync 1, %0;" ::"n"(NEPI) : "memory");
     }
@@ -521,22 +542,29 @@ size_t chunk_bytes() {
 
 int launch_gram(const void* prep, int m, int n, const int* idx, long long nsets, int k, float* blocks,
                 int* gerr, int* status, cudaStream_t st) {
+  // by lkp - 4
+  static decltype(&k_gram<7>) const kerns[4] = {k_gram<4>, k_gram<5>, k_gram<6>, k_gram<7>};
   static bool attr = [] {
-    cudaFuncSetAttribute(k_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+    for (auto kern : kerns)
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
     return true;
   }();
   (void)attr;
   const int kc_total = (m + KCH - 1) / KCH;
-  long long grid = api_device_sms();
-  if (nsets < grid) grid = nsets;
+  // as many sets per tile as k allows while every SM still gets a tile
+  int lkp = 7;
+  const long long sms = api_device_sms();
+  while (lkp > 4 && k <= (1 << (lkp - 1)) && (nsets >> (8 - lkp)) >= sms) --lkp;
+  const long long ntiles = (nsets + (1 << (7 - lkp)) - 1) >> (7 - lkp);
+  const long long grid = ntiles < sms ? ntiles : sms;
   // PL_GRAM_TEST_HOLD=1 (tests of the timeout path only): the MMA thread
   // issues nothing, every bounded wait of the other roles gives up after 2 s,
   // the kernel frees its TMEM and returns, and the call reports PL_ETIMEDOUT.
   const char* h = getenv("PL_GRAM_TEST_HOLD");
   const int hold = (h && h[0] == '1') ? 1 : 0;
   const float* nrm2 = (const float*)((const char*)prep + (size_t)n * kc_total * REC_BYTES);
-  k_gram<<<(unsigned)grid, NTHREADS, kSmemBytes, st>>>((const char*)prep, nrm2, n, kc_total, idx, nsets,
-                                                       k, blocks, gerr, status, hold);
+  kerns[lkp - 4]<<<(unsigned)grid, NTHREADS, kSmemBytes, st>>>((const char*)prep, nrm2, n, kc_total, idx, nsets,
+                                                                k, blocks, gerr, status, hold);
   GCU(cudaGetLastError());
   return PL_OK;
 }
