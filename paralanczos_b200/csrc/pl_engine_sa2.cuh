@@ -121,18 +121,32 @@ __device__ __forceinline__ int solve_set_sa2(const MatrixF32& M, const int* __re
       const int r0 = p, r1 = KB - 1 - p;
       const float* __restrict__ row0 = SM.A + (size_t)sm.idx[r0] * (size_t)SM.lda;
       const float* __restrict__ row1 = SM.A + (size_t)sm.idx[r1] * (size_t)SM.lda;
-#pragma unroll 16
-      for (int ii = 0; ii < PER; ++ii) {
-        const int i = i0 + ii;
-        if (TPP > 1 && i > KB) break;
-        const bool first = i < KB - p;
-        const int r = first ? r0 : r1;
-        const int c = first ? p + i : i - 1;  // c >= r
-        const float e = (r < k && c < k) ? __ldg((first ? row0 : row1) + sm.idx[c]) : 0.f;
-        const double e2 = (double)e * (double)e;
-        fro += (c == r) ? e2 : 2.0 * e2;
-        Af[sa2_at<KB, RPT>(r, c)] = e;
-        if (c != r) Af[sa2_at<KB, RPT>(c, r)] = e;
+      // U loads at a time, then their stores: a store to A could alias the
+      // indices that the next load's address needs, and one load was in flight
+      constexpr int U = PER < 36 ? PER : (PER + 1) / 2;
+      for (int ii = 0; ii < PER; ii += U) {
+        float e[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int i = i0 + ii + u;
+          const bool first = i < KB - p;
+          const int r = first ? r0 : r1;
+          const int c = first ? p + i : i - 1;  // c >= r
+          const bool in = ii + u < PER && i <= KB && r < k && c < k;
+          e[u] = in ? __ldg((first ? row0 : row1) + sm.idx[in ? c : 0]) : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int i = i0 + ii + u;
+          if (ii + u >= PER || i > KB) break;
+          const bool first = i < KB - p;
+          const int r = first ? r0 : r1;
+          const int c = first ? p + i : i - 1;
+          const double e2 = (double)e[u] * (double)e[u];
+          fro += (c == r) ? e2 : 2.0 * e2;
+          Af[sa2_at<KB, RPT>(r, c)] = e[u];
+          if (c != r) Af[sa2_at<KB, RPT>(c, r)] = e[u];
+        }
       }
     }
   }

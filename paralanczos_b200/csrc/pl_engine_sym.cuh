@@ -61,6 +61,20 @@ __device__ __forceinline__ double sym_sum(const double* p) {
   return s;
 }
 
+// Row `lane` of block I of a product: its tile sums in block order (loaded
+// together; the order of the adds is the sum's).
+template <int NB>
+__device__ __forceinline__ float sym_row_sum(const float (&ys)[NB][NB][32], int I, int nb, int lane) {
+  float e[NB];
+#pragma unroll
+  for (int J = 0; J < NB; ++J) e[J] = J < nb ? ys[I][J][lane] : 0.f;
+  float y = 0.f;
+#pragma unroll
+  for (int J = 0; J < NB; ++J)
+    if (J < nb) y += e[J];
+  return y;
+}
+
 // Slot (a, s) of lane (rg, cg): tile row and column.
 __device__ __forceinline__ int sym_row(int rg, int cg, int a) { return 4 * rg + (a ^ (cg & 2)); }
 __device__ __forceinline__ int sym_col(int rg, int cg, int s) { return 8 * cg + (s ^ (rg & 6)); }
@@ -202,22 +216,33 @@ __device__ __forceinline__ void sym_solve_set(const MatrixF32& M, const int* __r
   for (int u = 0; u < TPW; ++u) {
     const bool act = TJ[u] < nb;
     const bool diag = TI[u] == TJ[u];
+    // (a tile's 32 loads before its stores: a store to A could alias the indices
+    // that the next load's address needs)
+    float e[4][8];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      const int r = 32 * TI[u] + sym_row(rg, cg, a);
+      const bool rv = act && r < k;
+      const float* __restrict__ row = SM.A + (size_t)sm.idx[rv ? r : 0] * (size_t)SM.lda;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int c = 32 * TJ[u] + sym_col(rg, cg, q);
+        e[a][q] = (rv && c < k) ? __ldg(row + sm.idx[c]) : 0.f;
+      }
+    }
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
       const int rl = sym_row(rg, cg, a), r = 32 * TI[u] + rl;
       const bool rv = act && r < k;
-      const float* __restrict__ row = SM.A + (size_t)sm.idx[rv ? r : 0] * (size_t)SM.lda;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        float e[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const int c = 32 * TJ[u] + sym_col(rg, cg, 4 * h + q);
-          e[q] = (rv && c < k) ? __ldg(row + sm.idx[c]) : 0.f;
-          const double e2 = (double)e[q] * (double)e[q];
+          const double e2 = (double)e[a][4 * h + q] * (double)e[a][4 * h + q];
           fro += diag ? e2 : 2.0 * e2;
         }
-        if (act) sm.A[TT[u]][2 * a + h][lane] = make_float4(e[0], e[1], e[2], e[3]);
+        if (act)
+          sm.A[TT[u]][2 * a + h][lane] = make_float4(e[a][4 * h], e[a][4 * h + 1], e[a][4 * h + 2], e[a][4 * h + 3]);
 #pragma unroll
         for (int p = 0; p < 2; ++p) {
           const int cl = sym_col(rg, cg, 4 * h + 2 * p);  // cl + 1 is slot 4h + 2p + 1's column
@@ -300,13 +325,11 @@ __device__ __forceinline__ void sym_solve_set(const MatrixF32& M, const int* __r
 
     // ---- B: alpha, w~ = y - alpha v_j - beta_j v_{j-1} (the row warps) ---------
     if (t < KB) {
-      const double alpha = sym_sum<NW>(sm.pa);
-      const float af = (float)alpha;
       const int I = t >> 5;
-      float y = 0.f;
-      if (I < nb)
-        for (int J = 0; J < nb; ++J) y += sm.ys[I][J][lane];
-      sm.wt[t] = fmaf(-af, sc * sm.wb[cur][t], fmaf(-bprev, scp * sm.wb[prv][t], y));
+      const float y = I < nb ? sym_row_sum<NB>(sm.ys, I, nb, lane) : 0.f;
+      const float yp = fmaf(-bprev, scp * sm.wb[prv][t], y), vc = sc * sm.wb[cur][t];
+      const double alpha = sym_sum<NW>(sm.pa);
+      sm.wt[t] = fmaf(-(float)alpha, vc, yp);
       if (t == 0) sm.ab[j].x = alpha;
     }
     if (j + 1 == k) break;  // a non-finite alpha shows in ||w||^2 (or, at the end, in T)
@@ -319,9 +342,7 @@ __device__ __forceinline__ void sym_solve_set(const MatrixF32& M, const int* __r
     // ---- D: w, ||w||^2 ------------------------------------------------------------
     if (t < KB) {
       const int I = t >> 5;
-      float wv = 0.f;
-      if (I < nb)
-        for (int J = 0; J < nb; ++J) wv += sm.ys[I][J][lane];
+      const float wv = I < nb ? sym_row_sum<NB>(sm.ys, I, nb, lane) : 0.f;
       sm.wb[nxt][t] = wv;
       const double bp = warp_sum((double)wv * (double)wv);
       if (lane == 0) sm.pb[w] = bp;
@@ -379,9 +400,7 @@ __device__ __forceinline__ void sym_solve_set(const MatrixF32& M, const int* __r
       __syncthreads();
       if (t < KB) {
         const int I = t >> 5;
-        float z = 0.f;
-        if (I < nb)
-          for (int J = 0; J < nb; ++J) z += sm.ys[I][J][lane];
+        const float z = I < nb ? sym_row_sum<NB>(sm.ys, I, nb, lane) : 0.f;
         sm.wb[nxt][t] = z;
         const double zp = warp_sum((double)z * (double)z);
         if (lane == 0) sm.pz[w] = zp;
