@@ -849,7 +849,7 @@ static uint64_t hash_doubles(const double* p, size_t n) {
 // solve starts on the cached copy at once and the contents are hashed on the
 // host while it runs; a changed hash re-uploads the matrix and solves again
 // before anything is copied back.  Synchronous on the legacy default stream,
-// like the reference.
+// like the reference.  A matrix not cached is hashed during its first solve too.
 int api_solve_f64_host(const double* mat, int n, const int* subIndex, long long nsets, int k, int form,
                        double* eig, double* det, int* err) {
   std::lock_guard<std::mutex> lk(g_mu);
@@ -859,7 +859,8 @@ int api_solve_f64_host(const double* mat, int n, const int* subIndex, long long 
   cudaStream_t st = 0;
   const size_t nn = (size_t)n * (size_t)n;
   static const bool cache_on = env_flag("PL_DROPIN_CACHE", true);
-  auto upload = [&](uint64_t h) -> int {
+  // (the matrix counts as cached once its contents are hashed, below)
+  auto upload = [&]() -> int {
     d.mc.valid = false;
     int rc = ensure(d.mat64, sizeof(double) * nn);
     if (rc) return rc;
@@ -870,16 +871,18 @@ int api_solve_f64_host(const double* mat, int n, const int* subIndex, long long 
     k_f64_to_f32<<<(unsigned)(g < 8192 ? g : 8192), 256, 0, st>>>((const double*)d.mat64.p, (float*)d.mat32.p,
                                                                 (long long)nn);
     PL_CU(cudaGetLastError());
+    ++d.mc.misses;
+    return PL_OK;
+  };
+  auto cached = [&](uint64_t h) {
     d.mc.host = mat;
     d.mc.n = n;
     d.mc.hash = h;
     d.mc.valid = cache_on;
-    ++d.mc.misses;
-    return PL_OK;
   };
   const bool speculate = cache_on && d.mc.valid && d.mc.host == mat && d.mc.n == n;
   if (!speculate) {
-    const int rc = upload(cache_on ? hash_doubles(mat, nn) : 0);
+    const int rc = upload();
     if (rc) return rc;
   }
   const long long total = nsets * (long long)k;
@@ -896,15 +899,18 @@ int api_solve_f64_host(const double* mat, int n, const int* subIndex, long long 
   SetOutputs out{nullptr, nullptr, nullptr, derr, deig, ddet};
   rc = solve_dev((const float*)d.mat32.p, n, n, dI, nullptr, nsets, k, form, out, st);
   if (rc) return rc;
-  if (speculate) {
+  if (cache_on) {
     const uint64_t h = hash_doubles(mat, nn);  // overlaps the solve
-    if (h == d.mc.hash) {
+    if (!speculate) {
+      cached(h);
+    } else if (h == d.mc.hash) {
       ++d.mc.hits;
     } else {
-      rc = upload(h);
+      rc = upload();
       if (rc) return rc;
       rc = solve_dev((const float*)d.mat32.p, n, n, dI, nullptr, nsets, k, form, out, st);
       if (rc) return rc;
+      cached(h);
     }
   }
   if (eig) PL_CU(cudaMemcpyAsync(eig, deig, sizeof(double) * total, cudaMemcpyDeviceToHost, st));
