@@ -202,24 +202,46 @@ __device__ __forceinline__ int solve_set_sa(const MatrixF32& M, const int* __res
       const int r0 = p, r1 = KB - 1 - p;
       const float* __restrict__ row0 = SM.A + (size_t)sm.idx[r0] * (size_t)SM.lda;
       const float* __restrict__ row1 = SM.A + (size_t)sm.idx[r1] * (size_t)SM.lda;
-#pragma unroll 8
-      for (int ii = 0; ii < PER; ++ii) {
-        const int i = i0 + ii;
-        if (TPP > 1 && i > KB) break;
-        const bool first = i < KB - p;
-        const int r = first ? r0 : r1;
-        const int c = first ? p + i : i - 1;  // c >= r
-        float e = 0.f;
-        if (r < k && c < k) {
-          if (PF && have)
-            e = stg->e[ii * NT + t];
-          else
-            e = __ldg((first ? row0 : row1) + sm.idx[c]);
+      if (PF && have) {
+        // from the stage, U elements at a time: read ahead of their stores, which
+        // could alias the next reads (one at a time took 230 cycles an element)
+        constexpr int U = 13;
+        double fa = 0.0, fb = 0.0;  // diagonal, upper triangle
+        for (int ii = 0; ii < PER; ii += U) {
+          float e[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) e[u] = stg->e[(ii + u < PER ? ii + u : 0) * NT + t];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int i = i0 + ii + u;
+            const bool first = i < KB - p;
+            const int r = first ? r0 : r1;
+            const int c = first ? p + i : i - 1;  // c >= r
+            if (ii + u < PER && i <= KB) {
+              const float x = (r < k && c < k) ? e[u] : 0.f;
+              const double e2 = (double)x * (double)x;
+              if (c == r) fa += e2; else fb += e2;
+              Af[sa_at<NT, NCH>(r, c)] = x;
+              if (c != r) Af[sa_at<NT, NCH>(c, r)] = x;
+            }
+          }
         }
-        const double e2 = (double)e * (double)e;
-        fro += (c == r) ? e2 : 2.0 * e2;
-        Af[sa_at<NT, NCH>(r, c)] = e;
-        if (c != r) Af[sa_at<NT, NCH>(c, r)] = e;
+        fro = fa + 2.0 * fb;
+      } else {
+#pragma unroll 8
+        for (int ii = 0; ii < PER; ++ii) {
+          const int i = i0 + ii;
+          if (TPP > 1 && i > KB) break;
+          const bool first = i < KB - p;
+          const int r = first ? r0 : r1;
+          const int c = first ? p + i : i - 1;  // c >= r
+          float e = 0.f;
+          if (r < k && c < k) e = __ldg((first ? row0 : row1) + sm.idx[c]);
+          const double e2 = (double)e * (double)e;
+          fro += (c == r) ? e2 : 2.0 * e2;
+          Af[sa_at<NT, NCH>(r, c)] = e;
+          if (c != r) Af[sa_at<NT, NCH>(c, r)] = e;
+        }
       }
 #pragma unroll
       for (int q = 0; q < RPT; ++q) {
