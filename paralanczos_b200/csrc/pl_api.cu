@@ -405,9 +405,6 @@ struct Variant {
         {scratch_large<KM>, scratch_large<KM>}                                           \
   }
 
-// most sets per SM of a short call (short_call below)
-constexpr int kShortSetsPerSm = 16;
-
 const int kBinK[] = {8, 16, 32, 48, 64, 96, 128, 192, 256, 384, 512};
 constexpr int kNumBins = 11;
 
@@ -461,6 +458,23 @@ const Variant& chosen_for(int b, bool all) {
   if (v.fn[all ? 1 : 0]) return v;
   for (const Variant& w : variants(b))
     if (w.fn[all ? 1 : 0]) return w;
+  return v;
+}
+
+// The same for a call of nsets sets.  All eigenvalues at 48 < k <= 64 by the
+// tensor-memory kernel (8 sets an SM at once, one warp each): a few sets take
+// 6/5 of the time of the register kernel's (6 sets an SM, two warps each), so
+// that one runs where its waves are the cheaper ones (k = 64: 300 sets 112 -> 96
+// us, 2,400 391 -> 335; 4,800 665 -> 648; but 900, two waves against one, 146
+// against 191, and 10,000 1,201 against 1,281).  Neither needs scratch; their
+// FP32 sums are the same, their FP64 sums differ in the last bits.
+const Variant& variant_for(int b, bool all, long long nsets) {
+  const Variant& v = chosen_for(b, all);
+  if (kBinK[b] == 64 && all && g_variant[b] == 10 && nsets >= 0) {
+    const long long sms = device_sms();
+    const long long reg = (nsets + 6 * sms - 1) / (6 * sms), tmem = (nsets + 8 * sms - 1) / (8 * sms);
+    if (5 * reg <= 6 * tmem) return variants(b)[0];
+  }
   return v;
 }
 
@@ -556,16 +570,6 @@ bool env_flag(const char* name, bool dflt) {
   return !(v[0] == '0' || v[0] == 'n' || v[0] == 'N' || v[0] == 'f' || v[0] == 'F');
 }
 
-// A short call of 8 < k <= 16 runs on the next bin's kernel, one warp per set
-// instead of a quarter: its sums over a whole warp and its bisection by 16
-// threads per extreme are the shorter dependent chains, and the sets have the
-// SMs to themselves (the FP32 sums are the same: padding adds zeros).
-// 256 sets of k = 16: 30.3 -> 18.6 us on the GPU; equal at 16 sets per SM (28.9),
-// 33 against 41 at 28.
-bool short_call(int b, bool all, long long nsets) {
-  return kBinK[b] == 16 && !all && nsets <= (long long)device_sms() * kShortSetsPerSm;
-}
-
 // Uniform k: one kernel.
 int solve_uniform(const MatrixF32& M, const int* idx, long long nsets, int k, int form,
                   const SetOutputs& out, cudaStream_t st) {
@@ -577,8 +581,7 @@ int solve_uniform(const MatrixF32& M, const int* idx, long long nsets, int k, in
   }
   int b = bin_of_k(k);
   if (b < 0) return PL_ENOTSUP;
-  if (short_call(b, all, nsets)) ++b;
-  const Variant& v = chosen_for(b, all);
+  const Variant& v = variant_for(b, all, nsets);
   void* scratch = nullptr;
   const size_t need = v.scratch[all ? 1 : 0]();
   if (need) {
@@ -602,10 +605,10 @@ size_t binned_qscratch(int form, bool all, size_t off[kNumBins]) {
   return total;
 }
 
-void binned_fns(int form, bool all, LaunchFn fns[kNumBins]) {
+void binned_fns(int form, bool all, long long nsets, LaunchFn fns[kNumBins]) {
   for (int b = 0; b < kNumBins; ++b)
     fns[b] = (form == PL_FORM_PLAIN && kBinK[b] <= 128) ? plain_fn(kBinK[b], all)
-                                                        : chosen_for(b, all).fn[all ? 1 : 0];
+                                                        : variant_for(b, all, nsets).fn[all ? 1 : 0];
 }
 
 // The binned sequence on stream cs: count sets per k bin, scan, scatter the
@@ -679,7 +682,7 @@ int solve_csr(const MatrixF32& M, const int* idx, const long long* offsets, long
   auto it = d.graphs.find(key);
   if (it == d.graphs.end()) {
     LaunchFn fns[kNumBins];
-    binned_fns(form, all, fns);
+    binned_fns(form, all, nsets, fns);
     // load every kernel before the capture: nothing that may load a module
     // or set a function attribute runs while the stream is capturing
     for (int b = 0; b < kNumBins; ++b) PL_CU(fns[b](M, SetSource{}, out, 0, nullptr, d.side[b], true));
@@ -760,7 +763,7 @@ size_t api_binned_scratch(long long nsets, int form, bool all) {
 }
 int api_prepare_binned(int form, bool all) {
   LaunchFn fns[kNumBins];
-  binned_fns(form, all, fns);
+  binned_fns(form, all, -1, fns);
   SetOutputs out{};
   for (int b = 0; b < kNumBins; ++b) PL_CU(fns[b](MatrixF32{}, SetSource{}, out, 0, nullptr, 0, true));
   return PL_OK;
@@ -774,7 +777,7 @@ int api_launch_binned(const MatrixF32& M, const int* idx, const long long* offse
   size_t qoff[kNumBins];
   binned_qscratch(form, all, qoff);
   LaunchFn fns[kNumBins];
-  binned_fns(form, all, fns);
+  binned_fns(form, all, nsets_dev ? -1 : nsets, fns);
   char* base = (char*)scratch;
   int* hdr = (int*)base;
   char* q = base + align256(sizeof(int) * (48 + (size_t)nsets));

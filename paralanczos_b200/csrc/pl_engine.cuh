@@ -274,6 +274,7 @@ __device__ __forceinline__ int solve_set(const MatrixF32& M, const int* __restri
   }
   for (int c = t; c < KB; c += NT) sm.vb[c] = c < k ? v0 : 0.f;
   if (t == 0) sm.ab[0].y = 0.0;
+  if (t < 3 && k + t < KB) sm.ab[k + t] = sturm_pad_row(sqrt(fro2));
   float sc = 1.f;     // v = sc * vb (vb holds the unnormalised vector)
   float bprev = 0.f;  // beta_j for the three-term step
   int status = 0;
@@ -449,11 +450,11 @@ __device__ __forceinline__ int solve_set(const MatrixF32& M, const int* __restri
   {
     const int R = bisect_rounds(glo, ghi);
     double prod = 1.0;
-    // a thread's eigenvalues two at a time: their chains overlap
-    constexpr int EV = KB > NT ? 2 : 1;
+    // all of a thread's eigenvalues at once: their chains overlap
+    constexpr int EV = (KB + NT - 1) / NT;
     for (int m0 = t; m0 < k; m0 += EV * NT) {
       double lam[EV];
-      bisect_indices<(KB > 32 && KB <= 64 ? 16 : 8), EV>(sm.ab, k, m0, NT, glo, ghi, R, lam);
+      bisect_indices<(KB == 48 || KB == 64 ? 16 : 8), EV>(sm.ab, (k + 3) & ~3, m0, NT, glo, ghi, R, lam);
 #pragma unroll
       for (int v = 0; v < EV; ++v) {
         const int m = m0 + v * NT;

@@ -176,6 +176,7 @@ __device__ __forceinline__ int solve_set_sa2(const MatrixF32& M, const int* __re
   }
   for (int c = t; c < KB; c += NT) sm.vb[c] = c < k ? v0 : 0.f;
   if (t == 0) sm.ab[0].y = 0.0;
+  if (t < 3 && k + t < KB) sm.ab[k + t] = sturm_pad_row(sqrt(fro2));
   float sc = 1.f, bprev = 0.f;
   int status = 0;
   g.sync();

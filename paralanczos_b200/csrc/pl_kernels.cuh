@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(CTA, MINB)
   const long long ng = (long long)gridDim.x * GPC;
   const long long nitems = item_count(src);
   const int pbase = src.perm_start ? *src.perm_start : 0;
-  double2* __restrict__ T = qbuf + ((size_t)blockIdx.x * GPC + gic) * (size_t)(Q * KB);
+  double2* __restrict__ T = queue_slots<KB, C::NT>(qbuf + (size_t)blockIdx.x * GPC * (Q * KB), gic);
   int nq = 0;
   for (long long it = (long long)gic * gridDim.x + blockIdx.x; it < nitems; it += ng) {
     long long set, off;
@@ -52,13 +52,13 @@ __global__ void __launch_bounds__(CTA, MINB)
     const int st = solve_set<KB, RPT, TPR, ALL>(M, src.idx + off, k, set, off, out, smem[gic], g);
     if constexpr (!ALL) {
       if (st >= 0) {
-        const int kq = qmeta[gic][nq].k;
-        for (int i = g.t; i < kq; i += C::NT) T[(size_t)i * Q + nq] = smem[gic].ab[i];
+        const int kq = (qmeta[gic][nq].k + 3) & ~3;  // with the rows that fill T up
+        for (int i = g.t; i < kq; i += C::NT) T[(size_t)i * kQueueStride<C::NT> + nq] = smem[gic].ab[i];
         if (g.t == 0) qmeta[gic][nq].status = st;
         ++nq;
         g.sync();
         if (nq == Q) {
-          queue_bisect<KB, C::NT>(T, Q, nq, qmeta[gic], g.t, out, g.mask, nullptr);
+          queue_bisect<KB, C::NT>(T, nq, qmeta[gic], g.t, out, g.mask, nullptr);
           g.sync();
           nq = 0;
         }
@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(CTA, MINB)
     }
   }
   if constexpr (!ALL) {
-    if (nq > 0) queue_bisect<KB, C::NT>(T, Q, nq, qmeta[gic], g.t, out, g.mask, smem[gic].ab);
+    if (nq > 0) queue_bisect<KB, C::NT>(T, nq, qmeta[gic], g.t, out, g.mask, smem[gic].ab);
   }
 }
 
@@ -90,7 +90,7 @@ __device__ __forceinline__ void sa_solve_body(const MatrixF32& M, const SetSourc
   const long long ng = (long long)gridDim.x * GPC;
   const long long nitems = item_count(src);
   const int pbase = src.perm_start ? *src.perm_start : 0;
-  double2* __restrict__ T = qbuf + ((size_t)blockIdx.x * GPC + gic) * (size_t)(Q * KB);
+  double2* __restrict__ T = queue_slots<KB, C::NT>(qbuf + (size_t)blockIdx.x * GPC * (Q * KB), gic);
   // PF: the next set's triangle is staged behind this set's steps (SAStage
   // after the GPC SASmem slots)
   SAStage<KB, C::NT>* stg = PF ? reinterpret_cast<SAStage<KB, C::NT>*>(smem + GPC) + gic : nullptr;
@@ -130,13 +130,13 @@ __device__ __forceinline__ void sa_solve_body(const MatrixF32& M, const SetSourc
     have = issued;
     if constexpr (!ALL) {
       if (st >= 0) {
-        const int kq = qmeta[gic][nq].k;
-        for (int i = g.t; i < kq; i += C::NT) T[(size_t)i * Q + nq] = smem[gic].ab[i];
+        const int kq = (qmeta[gic][nq].k + 3) & ~3;  // with the rows that fill T up
+        for (int i = g.t; i < kq; i += C::NT) T[(size_t)i * kQueueStride<C::NT> + nq] = smem[gic].ab[i];
         if (g.t == 0) qmeta[gic][nq].status = st;
         ++nq;
         g.sync();
         if (nq == Q) {
-          queue_bisect<KB, C::NT>(T, Q, nq, qmeta[gic], g.t, out, g.mask, nullptr);
+          queue_bisect<KB, C::NT>(T, nq, qmeta[gic], g.t, out, g.mask, nullptr);
           g.sync();
           nq = 0;
         }
@@ -144,7 +144,7 @@ __device__ __forceinline__ void sa_solve_body(const MatrixF32& M, const SetSourc
     }
   }
   if constexpr (!ALL) {
-    if (nq > 0) queue_bisect<KB, C::NT>(T, Q, nq, qmeta[gic], g.t, out, g.mask, smem[gic].ab);
+    if (nq > 0) queue_bisect<KB, C::NT>(T, nq, qmeta[gic], g.t, out, g.mask, smem[gic].ab);
   }
   if constexpr (PF) cp_async_wait_all();  // no copy outlives the kernel
   am.end();
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(CTA, MINB)
   const long long ng = (long long)gridDim.x * GPC;
   const long long nitems = item_count(src);
   const int pbase = src.perm_start ? *src.perm_start : 0;
-  double2* __restrict__ T = qbuf + ((size_t)blockIdx.x * GPC + gic) * (size_t)(Q * KB);
+  double2* __restrict__ T = queue_slots<KB, C::NT>(qbuf + (size_t)blockIdx.x * GPC * (Q * KB), gic);
   int nq = 0;
   for (long long it = (long long)gic * gridDim.x + blockIdx.x; it < nitems; it += ng) {
     long long set, off;
@@ -206,19 +206,19 @@ __global__ void __launch_bounds__(CTA, MINB)
     if (g.t == 0) qmeta[gic][nq] = QueueMeta{set, k, 0};
     const int st = solve_set_sa2<KB, RPT, NB>(M, src.idx + off, k, set, off, out, smem[gic], g, am.ta);
     if (st >= 0) {
-      const int kq = qmeta[gic][nq].k;
-      for (int i = g.t; i < kq; i += C::NT) T[(size_t)i * Q + nq] = smem[gic].ab[i];
+      const int kq = (qmeta[gic][nq].k + 3) & ~3;  // with the rows that fill T up
+      for (int i = g.t; i < kq; i += C::NT) T[(size_t)i * kQueueStride<C::NT> + nq] = smem[gic].ab[i];
       if (g.t == 0) qmeta[gic][nq].status = st;
       ++nq;
       g.sync();
       if (nq == Q) {
-        queue_bisect<KB, C::NT>(T, Q, nq, qmeta[gic], g.t, out, g.mask, nullptr);
+        queue_bisect<KB, C::NT>(T, nq, qmeta[gic], g.t, out, g.mask, nullptr);
         g.sync();
         nq = 0;
       }
     }
   }
-  if (nq > 0) queue_bisect<KB, C::NT>(T, Q, nq, qmeta[gic], g.t, out, g.mask, smem[gic].ab);
+  if (nq > 0) queue_bisect<KB, C::NT>(T, nq, qmeta[gic], g.t, out, g.mask, smem[gic].ab);
   am.end();
 }
 

@@ -7,14 +7,26 @@
 // bisects them all at once, with one thread per extreme when the queue is full:
 // plain bisection, one bit per Sturm count, every lane doing distinct useful work.
 //
-// Buffer layout of one group: T[i][slot] (double2 {alpha_i, beta_i^2}), so the
-// lanes of a warp reading element i of their slots touch contiguous memory.
+// Buffer layout: T[i][slot] (double2 {alpha_i, beta_i^2}), the slots of all groups
+// of a warp side by side, so the lanes of a warp reading element i of their slots
+// touch contiguous memory (four groups' slots apart took four lines an element).
 #pragma once
 #include "pl_common.cuh"
 #include "pl_sturm.cuh"
 #include "pl_engine.cuh"
 
 namespace pl {
+
+// double2 between elements i and i + 1 of a slot.
+template <int NT>
+constexpr int kQueueStride = NT < 32 ? 16 : NT / 2;
+
+// Slots of group gic in the queue buffer of its CTA.
+template <int KB, int NT>
+__device__ __forceinline__ double2* queue_slots(double2* cta, int gic) {
+  constexpr int GPW = NT < 32 ? 32 / NT : 1, Q = NT / 2;
+  return cta + (size_t)(gic / GPW * GPW) * (Q * KB) + gic % GPW * Q;
+}
 
 struct QueueMeta {
   long long set;
@@ -29,7 +41,7 @@ struct QueueMeta {
 // 2^D - 1 midpoints that those levels can reach and take the interval of the
 // last one on the way, so the result is plain bisection's, in 1 / D of the
 // rounds.  A full queue has L = 1 (every thread an extreme of its own, D = 1);
-// a queue of few sets, as in a short call, would otherwise leave most threads
+// a queue of few sets, as in a call of few, would otherwise leave most threads
 // idle through some 36 serial rounds (one set of k = 32: 36,600 -> 12,000
 // cycles).  Groups of less than a warp always have L = 1: what the rounds save
 // their sub-warp shuffles cost (about 80 cycles each).  last: the T of the last
@@ -37,9 +49,9 @@ struct QueueMeta {
 // nullptr: no).  Every thread of the group must call it (mask: its lanes of the
 // warp).
 template <int KB, int NT>
-__device__ __forceinline__ void queue_bisect(const double2* __restrict__ T, int Q, int nslots,
-                                             const QueueMeta* __restrict__ meta, int t,
-                                             const SetOutputs& out, unsigned mask, const double2* last) {
+__device__ __forceinline__ void queue_bisect(const double2* __restrict__ T, int nslots,
+                                             const QueueMeta* __restrict__ meta, int t, const SetOutputs& out,
+                                             unsigned mask, const double2* last) {
   int L = 1, D = 1;
   if constexpr (NT >= 32) {
     if (NT / (2 * nslots) >= 4) {
@@ -57,19 +69,19 @@ __device__ __forceinline__ void queue_bisect(const double2* __restrict__ T, int 
   long long set = -1;
   double a = 0.0, b = 0.0;
   const double2* ab = T + (active ? slot : 0);
-  int stride = Q;
-  if (nslots == 1 && last) {
+  int stride = kQueueStride<NT>;
+  if (NT >= 32 && nslots == 1 && last) {
     ab = last;
     stride = 1;
   }
-  [[maybe_unused]] double2 tr[8];
+  [[maybe_unused]] double2 tr[KB <= 16 ? KB : 1];
   if (active) {
     k = meta[slot].k;
     status = meta[slot].status;
     set = meta[slot].set;
     if constexpr (KB == 8) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) tr[i] = ab[(size_t)(i < k ? i : k - 1) * stride];
+      for (int i = 0; i < 8; ++i) tr[i] = ab[(size_t)i * stride];
     }
   }
   const bool solve = active && !(status & SET_NONFINITE);
@@ -108,15 +120,25 @@ __device__ __forceinline__ void queue_bisect(const double2* __restrict__ T, int 
   }
   const int target = (e & 1) ? k : 1;
   auto count = [&](double x) -> int {
-    if constexpr (KB == 8) {
+    if constexpr (KB <= 16) {
+      // all rows loaded at fixed offsets (KB = 8: once, into registers), no
+      // branch but one: 1,160 -> 710 cycles a round of four k = 16 sets on a full
+      // SM, where the loads' wavefronts and the instruction issue bound it
       double p0 = 0.0, p1 = 1.0;
       unsigned sp = 0;
       int cnt = 0;
-      sturm_rows<8>(tr, k, x, p0, p1, sp, cnt);
+      if constexpr (KB == 16) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) tr[i] = ab[(size_t)i * kQueueStride<NT>];
+      }
+      if (k <= KB - 4)
+        sturm_rows<KB - 4, true>(tr, x, p0, p1, sp, cnt);
+      else
+        sturm_rows<KB, true>(tr, x, p0, p1, sp, cnt);
       return cnt;
     } else {
       // (blocks of 16 need 96 registers: the kernels with more than 128)
-      return sturm_count_strided<(KB == 32 ? 8 : 16)>(ab, stride, k, x);
+      return sturm_count_strided<(KB == 32 ? 8 : 16)>(ab, stride, (k + 3) & ~3, x);
     }
   };
   if (L == 1) {

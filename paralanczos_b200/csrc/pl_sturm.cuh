@@ -23,32 +23,66 @@ __device__ __forceinline__ void sturm_rescale(double& p0, double& p1) {
   p1 *= s;
 }
 
-// U rows of the minors' recurrence at once: p_i = (alpha_i - x) p_{i-1} -
-// beta_i^2 p_{i-2}.  The signs are looked at only when the U minors are done
-// (the empty asm holds that work behind them): an integer use of a minor right
-// behind it stalls the chain.  Rows r .. U - 1 do not count.
-template <int U>
-__device__ __forceinline__ void sturm_rows(const double2 (&t)[U], int r, double x, double& p0, double& p1,
-                                           unsigned& sp, int& cnt) {
-  static_assert(U == 8 || U == 16, "rows per block");
-  double p[U];
+// N rows of the minors' recurrence, p_i = (alpha_i - x) p_{i-1} - beta_i^2 p_{i-2},
+// behind p1 = p_{i-1} and p0 = p_{i-2}; FIRST: rows 0 .. N - 1, whose first two
+// need no products with p_{-1} = 0 and p_0 = 1.
+template <int N, bool FIRST>
+__device__ __forceinline__ void sturm_minors(const double2* t, double x, double& p0, double& p1, double* p) {
 #pragma unroll
-  for (int u = 0; u < U; ++u) {
-    const double pm1 = u == 0 ? p1 : p[u > 0 ? u - 1 : 0];
-    const double pm2 = u == 0 ? p0 : (u == 1 ? p1 : p[u > 1 ? u - 2 : 0]);
-    p[u] = fma(t[u].x - x, pm1, -t[u].y * pm2);
+  for (int u = 0; u < N; ++u) {
+    const double d = t[u].x - x;
+    if (FIRST && u == 0) {
+      p[u] = d;
+    } else if (FIRST && u == 1) {
+      p[u] = fma(d, p[0], -t[u].y);
+    } else {
+      const double pm1 = u == 0 ? p1 : p[u > 0 ? u - 1 : 0];
+      const double pm2 = u == 0 ? p0 : (u == 1 ? p1 : p[u > 1 ? u - 2 : 0]);
+      p[u] = fma(d, pm1, -t[u].y * pm2);
+    }
   }
-  if constexpr (U == 16)
-    asm volatile("" : "+d"(p[8]), "+d"(p[9]), "+d"(p[10]), "+d"(p[11]), "+d"(p[12]), "+d"(p[13]), "+d"(p[14]),
-                      "+d"(p[15]));
-  asm volatile("" : "+d"(p[0]), "+d"(p[1]), "+d"(p[2]), "+d"(p[3]), "+d"(p[4]), "+d"(p[5]), "+d"(p[6]), "+d"(p[7]));
+  p0 = N > 1 ? p[N > 1 ? N - 2 : 0] : (FIRST ? 1.0 : p1);
+  p1 = p[N - 1];
+}
+
+// N rows at once.  The signs are looked at only when the N minors are done (the
+// empty asm holds that work behind them): an integer use of a minor right
+// behind it stalls the chain.
+template <int N, bool FIRST>
+__device__ __forceinline__ void sturm_rows(const double2* t, double x, double& p0, double& p1, unsigned& sp,
+                                           int& cnt) {
+  static_assert(N == 4 || N == 8 || N == 12 || N == 16, "rows per block");
+  double p[N];
+  sturm_minors<N, FIRST>(t, x, p0, p1, p);
+#pragma unroll
+  for (int u = N - 4; u >= 0; u -= 4)
+    asm volatile("" : "+d"(p[u]), "+d"(p[u + 1]), "+d"(p[u + 2]), "+d"(p[u + 3]));
   unsigned m = sp;  // signs, the newest in bit 0
 #pragma unroll
-  for (int u = 0; u < U; ++u) m = __funnelshift_l((unsigned)__double2hiint(p[u]), m, 1);
-  cnt += __popc((m ^ (m >> 1)) & (((1u << U) - 1u) & ~((1u << (U - r)) - 1u)));
+  for (int u = 0; u < N; ++u) m = __funnelshift_l((unsigned)__double2hiint(p[u]), m, 1);
+  cnt += __popc((m ^ (m >> 1)) & ((1u << N) - 1u));
   sp = m & 1u;
-  p0 = p[U - 2];
-  p1 = p[U - 1];
+}
+
+// A decoupled row above the spectrum: no sign change at any x in it.  The
+// engines whose T is counted many times over fill k up to a multiple of 4 with
+// such rows (fro: Frobenius norm of A_S; 2^-290: above the couplings of 2^-300
+// that a decoupled block stores, all that a zero matrix has), so that the counts
+// have no odd rows at the end (one at a time they cost 60 to 100 cycles each).
+__device__ __forceinline__ double2 sturm_pad_row(double fro) { return make_double2(4.0 * fro + 0x1p-290, 0.0); }
+
+// N rows from row i on for each x.
+template <int N, int E, bool FIRST>
+__device__ __forceinline__ void sturm_block(const double2* __restrict__ ab, int stride, int i, const double (&x)[E],
+                                            double (&p0)[E], double (&p1)[E], unsigned (&sp)[E], int (&cnt)[E]) {
+  double2 t[N];
+#pragma unroll
+  for (int u = 0; u < N; ++u) t[u] = ab[(size_t)(i + u) * stride];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    if (!FIRST && (i & 15) == 0) sturm_rescale(p0[e], p1[e]);
+    sturm_rows<N, FIRST>(t, x[e], p0[e], p1[e], sp[e], cnt[e]);
+  }
 }
 
 // Numbers of eigenvalues of T strictly below x[0 .. E-1].  Element i of T at
@@ -57,9 +91,10 @@ __device__ __forceinline__ void sturm_rows(const double2 (&t)[U], int r, double 
 // vanish).  Sign changes of the leading principal minors p_{-1} = 0, p_0 = 1,
 // ...; a minor that is exactly zero counts as positive, which gives the right
 // count because its neighbours then have opposite signs.  Rows go in blocks of
-// U, each loaded before its recurrence, the last one filled up with rows that
-// do not count; 25 to 30 cycles a row where loads and signs in the chain took 42
-// (one warp, B200).  E > 1 shares the loads and runs E chains side by side.
+// U, the last ones in a block of 12, 8 or 4 and one at a time, each block loaded
+// before its recurrence; 25 to 30 cycles a row where loads and signs in the chain
+// took 42 (one warp, B200).  E > 1 shares the loads and runs E chains side by
+// side.
 template <int U, int E>
 __device__ __forceinline__ void sturm_counts(const double2* __restrict__ ab, int stride, int k,
                                              const double (&x)[E], int (&cnt)[E]) {
@@ -73,24 +108,31 @@ __device__ __forceinline__ void sturm_counts(const double2* __restrict__ ab, int
     cnt[e] = 0;
   }
   int i = 0;
-  for (; i + U <= k; i += U) {
-    double2 t[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) t[u] = ab[(size_t)(i + u) * stride];
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      if (i > 0 && (i & 15) == 0) sturm_rescale(p0[e], p1[e]);
-      sturm_rows<U>(t, U, x[e], p0[e], p1[e], sp[e], cnt[e]);
-    }
+  if (k >= U) {
+    sturm_block<U, E, true>(ab, stride, 0, x, p0, p1, sp, cnt);
+    for (i = U; i + U <= k; i += U) sturm_block<U, E, false>(ab, stride, i, x, p0, p1, sp, cnt);
   }
-  if (i < k) {
-    double2 t[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) t[u] = ab[(size_t)(i + u < k ? i + u : k - 1) * stride];
+  const int r = k - i;
+  if (U > 8 && r >= 12) {
+    sturm_block<(U > 8 ? 12 : 4), E, false>(ab, stride, i, x, p0, p1, sp, cnt);
+    i += 12;
+  } else if (U > 8 && r >= 8) {
+    sturm_block<8, E, false>(ab, stride, i, x, p0, p1, sp, cnt);
+    i += 8;
+  } else if (r >= 4) {
+    sturm_block<4, E, false>(ab, stride, i, x, p0, p1, sp, cnt);
+    i += 4;
+  }
+  for (; i < k; ++i) {
+    const double2 t = ab[(size_t)i * stride];
 #pragma unroll
     for (int e = 0; e < E; ++e) {
-      if (i > 0 && (i & 15) == 0) sturm_rescale(p0[e], p1[e]);
-      sturm_rows<U>(t, k - i, x[e], p0[e], p1[e], sp[e], cnt[e]);
+      const double p2 = fma(t.x - x[e], p1[e], i > 0 ? -t.y * p0[e] : 0.0);
+      const unsigned s2 = (unsigned)__double2hiint(p2) >> 31;
+      cnt[e] += (int)(s2 ^ sp[e]);
+      sp[e] = s2;
+      p0[e] = p1[e];
+      p1[e] = p2;
     }
   }
 }
@@ -114,16 +156,17 @@ __device__ __forceinline__ double bisect_tol(double lo, double hi) {
   return 0x1p-34 * fmax(fabs(lo), fabs(hi)) + 1e-300;
 }
 
-// Rounds of bisection needed to shrink [lo, hi] below tol.
+// Rounds of bisection needed to shrink [lo, hi] below tol: the smallest r with
+// (hi - lo) 2^-r <= tol, read off the exponents and mantissas (halving in a loop
+// took 1,000 cycles).
 __device__ __forceinline__ int bisect_rounds(double lo, double hi) {
-  double w = hi - lo;
-  const double tol = bisect_tol(lo, hi);
-  int r = 0;
-  while (w > tol && r < 200) {
-    w *= 0.5;
-    ++r;
-  }
-  return r;
+  const double w = hi - lo;
+  const double tol = bisect_tol(lo, hi);  // >= 1e-300: normal
+  if (!(w > tol)) return 0;
+  const long long bw = __double_as_longlong(w), bt = __double_as_longlong(tol);
+  const long long mant = (1LL << 52) - 1;
+  const int r = (int)((bw >> 52) - (bt >> 52)) + ((bw & mant) > (bt & mant) ? 1 : 0);
+  return r < 200 ? r : 200;
 }
 
 // Rounds of (G+1)-way multisection needed to shrink [lo, hi] below tol.
