@@ -13,7 +13,7 @@
 // once per set and is streamed from there: the shared-memory pipe, at 59 % with
 // A_S in it, is the busiest unit.  Measured at k = 64 (B200, 200,000 sets): 11.7
 // M sets/s; with the FP64 sums on the matrix unit (warp_sum) 13.4 M; with A_S
-// in tensor memory 14.5 M.
+// in tensor memory 14.5 M; with the staged triangle mirrored in batches 15.3 M.
 //
 // A layout: thread t of a group of NT owns rows r_q = t + q*NT (q < RPT); its
 // row data is stored lane-interleaved, A[q][chunk][t][4] (4 floats per chunk),

@@ -15,9 +15,9 @@
 // triangle, and from there into tensor memory (pl_tmem.cuh), which every step
 // streams while the shared-memory pipe carries only the broadcasts and the
 // sums.  Measured (B200, 50,000 sets of a 4096-column matrix, sets/s): k = 96
-// 2.99e6 with A_S in shared memory and three warps per set, 3.87e6; k = 128
-// 1.36e6, 1.74e6 (of the latter's gain a third is the FP64 sums on the matrix
-// unit, warp_sum).
+// 2.99e6 with A_S in shared memory and three warps per set, 3.87e6, with the
+// gather in batches 4.0e6; k = 128 1.36e6, 1.74e6, 1.76e6 (of the first gain
+// there a third is the FP64 sums on the matrix unit, warp_sum).
 //
 // Layout of A_S in shared memory: element (r, c), r = rs + q * NR, chunk
 // cc = c / 4 = h + 2 ch, lives at float4 index (q * NCHT + ch) * NT + (rs * 2 + h):
