@@ -240,7 +240,7 @@ __device__ __forceinline__ void cgs_solve_set(const MatrixF32& M, const int* __r
     if constexpr (NW >= 2) {
       // warp 0 brackets lambda_min, warp 1 lambda_max, 33-way each
       if (g.wig < 2) {
-        const double e = multisect_warp(sm.ab, k, glo, ghi, g.wig == 0 ? 1 : k);
+        const double e = multisect_warp<true>(sm.ab, k, glo, ghi, g.wig == 0 ? 1 : k);
         if ((threadIdx.x & 31) == 0) sm.red[4 + g.wig][0] = e;
       }
       g.sync();

@@ -150,6 +150,31 @@ __device__ __forceinline__ int sturm_count(const double2* __restrict__ ab, int k
   return sturm_count_strided<8>(ab, 1, k, x);
 }
 
+// The same count a row at a time, in few registers: for the kernels of many
+// threads a set, where the blocks' registers cost more than the chain (plain
+// form, k = 64: 3.80e6 sets/s, 2.98e6 with blocks of 8).
+__device__ __forceinline__ int sturm_count_lean(const double2* __restrict__ ab, int k, double x) {
+  double p0 = 1.0, p1 = ab[0].x - x;
+  unsigned sp = (unsigned)__double2hiint(p1) >> 31;
+  int cnt = (int)sp;
+  auto row = [&](const double2 t) {
+    const double p2 = fma(t.x - x, p1, -t.y * p0);
+    const unsigned s2 = (unsigned)__double2hiint(p2) >> 31;
+    cnt += (int)(s2 ^ sp);
+    sp = s2;
+    p0 = p1;
+    p1 = p2;
+  };
+  int i = 1;
+  for (; i + 16 <= k; i += 16) {
+#pragma unroll
+    for (int u = 0; u < 16; ++u) row(ab[i + u]);
+    sturm_rescale(p0, p1);
+  }
+  for (; i < k; ++i) row(ab[i]);
+  return cnt;
+}
+
 // Termination width for an interval whose ends have magnitude up to `mag`.
 // 2^-34 (6e-11) of the spectrum's scale: far below the FP32 Lanczos error.
 __device__ __forceinline__ double bisect_tol(double lo, double hi) {
@@ -198,7 +223,7 @@ __device__ __forceinline__ void multisect_extremes(const double2* __restrict__ a
   for (int r = 0; r < R; ++r) {
     const double step = (b - a) / (double)(G + 1);
     const double x = a + step * (double)(gi + 1);
-    const bool pass = sturm_count(ab, k, x) >= target;
+    const bool pass = sturm_count_lean(ab, k, x) >= target;
     const unsigned bal = __ballot_sync(mask, pass);
     const unsigned mine = (bal >> shift) & gm;
     const int f = mine ? (__ffs(mine) - 1) : G;  // first sub-lane whose point passed
@@ -214,6 +239,7 @@ __device__ __forceinline__ void multisect_extremes(const double2* __restrict__ a
 
 // One extreme by (G+1)-way multisection with the G = 32 lanes of one warp:
 // the smallest x with count(x) >= target (target 1: lambda_min; k: lambda_max).
+template <bool LEAN = false>
 __device__ __forceinline__ double multisect_warp(const double2* __restrict__ ab, int k, double lo,
                                                  double hi, int target) {
   constexpr int G = 32;
@@ -223,7 +249,7 @@ __device__ __forceinline__ double multisect_warp(const double2* __restrict__ ab,
   for (int r = 0; r < R; ++r) {
     const double step = (b - a) / (double)(G + 1);
     const double x = a + step * (double)(gi + 1);
-    const unsigned bal = __ballot_sync(0xffffffffu, sturm_count(ab, k, x) >= target);
+    const unsigned bal = __ballot_sync(0xffffffffu, (LEAN ? sturm_count_lean(ab, k, x) : sturm_count(ab, k, x)) >= target);
     const int f = bal ? (__ffs(bal) - 1) : G;
     const double na = (f > 0) ? a + step * (double)f : a;
     const double nb = (f < G) ? a + step * (double)(f + 1) : b;
@@ -259,12 +285,14 @@ __device__ __forceinline__ void bisect_indices(const double2* __restrict__ ab, i
   for (int e = 0; e < E; ++e) lam[e] = 0.5 * (a[e] + b[e]);
 }
 
-// Eigenvalue number m.
+// Eigenvalue number m (m = 0 .. k - 1 on as many threads: counts in few registers).
 __device__ __forceinline__ double bisect_index(const double2* __restrict__ ab, int k, int m,
                                                double lo, double hi, int R) {
-  double lam[1];
-  bisect_indices<8, 1>(ab, k, m, 0, lo, hi, R, lam);
-  return lam[0];
+  for (int r = 0; r < R; ++r) {
+    const double x = 0.5 * (lo + hi);
+    if (sturm_count_lean(ab, k, x) >= m + 1) hi = x; else lo = x;
+  }
+  return 0.5 * (lo + hi);
 }
 
 }  // namespace pl
