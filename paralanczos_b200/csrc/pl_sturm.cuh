@@ -3,7 +3,7 @@
 // Replaces the reference's serial one-lane TQLRAT (ParaLanczos.cu:32-189, called
 // at ParaLanczos.cu:1461).  The count of eigenvalues of T below x is the number of
 // sign changes of the leading principal minors of T - xI (continuant form,
-// division-free, with power-of-two rescaling every 16 rows).  The reference's
+// division-free, with power-of-two rescaling every 8 or 16 rows).  The reference's
 // own Sturm sketch, EIGVALS_BELOW (ParaLanczos.cu:519-552), is unused and skips
 // alpha[1]; this is new code.  The CPU restatement is orc_sturm_count in
 // oracle/pl_oracle.c.
@@ -12,13 +12,14 @@
 
 namespace pl {
 
-// Power-of-two rescaling of the last two minors by p1's exponent: exact, keeps
-// signs and ratios.  (Without a branch: a taken-or-not one costs as much as ten
-// rows.)  A zero p1 leaves them as they are.
+// Power-of-two rescaling of the last two minors by p1's exponent, or by p0's
+// where p1 is zero or subnormal: exact, keeps signs and ratios.  (Without a
+// branch: a taken-or-not one costs as much as ten rows.)
 __device__ __forceinline__ void sturm_rescale(double& p0, double& p1) {
-  const int f = (__double2hiint(p1) >> 20) & 0x7ff;  // |p1| = m * 2^(f - 1023), m in [1, 2)
-  const int c = f < 2 ? 1023 : (f > 2043 ? 2043 : f);
-  const double s = __hiloint2double((f == 0 ? 1023 : 2046 - c) << 20, 0);  // 2^(1023 - c)
+  const int f1 = (__double2hiint(p1) >> 20) & 0x7ff;  // |p1| = m * 2^(f1 - 1023), m in [1, 2)
+  const int f = f1 < 2 ? (__double2hiint(p0) >> 20) & 0x7ff : f1;
+  const int c = f < 1 ? 1 : (f > 2043 ? 2043 : f);
+  const double s = __hiloint2double((2046 - c) << 20, 0);  // 2^(1023 - c)
   p0 *= s;
   p1 *= s;
 }
@@ -71,8 +72,8 @@ __device__ __forceinline__ void sturm_rows(const double2* t, double x, double& p
 // have no odd rows at the end (one at a time they cost 60 to 100 cycles each).
 __device__ __forceinline__ double2 sturm_pad_row(double fro) { return make_double2(4.0 * fro + 0x1p-290, 0.0); }
 
-// N rows from row i on for each x.
-template <int N, int E, bool FIRST>
+// N rows from row i on for each x, rescaled every RES rows.
+template <int N, int E, bool FIRST, int RES>
 __device__ __forceinline__ void sturm_block(const double2* __restrict__ ab, int stride, int i, const double (&x)[E],
                                             double (&p0)[E], double (&p1)[E], unsigned (&sp)[E], int (&cnt)[E]) {
   double2 t[N];
@@ -80,7 +81,7 @@ __device__ __forceinline__ void sturm_block(const double2* __restrict__ ab, int 
   for (int u = 0; u < N; ++u) t[u] = ab[(size_t)(i + u) * stride];
 #pragma unroll
   for (int e = 0; e < E; ++e) {
-    if (!FIRST && (i & 15) == 0) sturm_rescale(p0[e], p1[e]);
+    if (!FIRST && (i & (RES - 1)) == 0) sturm_rescale(p0[e], p1[e]);
     sturm_rows<N, FIRST>(t, x[e], p0[e], p1[e], sp[e], cnt[e]);
   }
 }
@@ -94,8 +95,10 @@ __device__ __forceinline__ void sturm_block(const double2* __restrict__ ab, int 
 // U, the last ones in a block of 12, 8 or 4 and one at a time, each block loaded
 // before its recurrence; 25 to 30 cycles a row where loads and signs in the chain
 // took 42 (one warp, B200).  E > 1 shares the loads and runs E chains side by
-// side.
-template <int U, int E>
+// side.  The minors are rescaled every RES rows, single rows among them: a run
+// of 16 rows stays within FP64 for matrices of scale 2^-59 to 2^57 or so, a run
+// of 19 (three single rows behind 16) did so only from 2^-52 to 2^53.
+template <int U, int E, int RES = 16>
 __device__ __forceinline__ void sturm_counts(const double2* __restrict__ ab, int stride, int k,
                                              const double (&x)[E], int (&cnt)[E]) {
   double p0[E], p1[E];
@@ -109,24 +112,25 @@ __device__ __forceinline__ void sturm_counts(const double2* __restrict__ ab, int
   }
   int i = 0;
   if (k >= U) {
-    sturm_block<U, E, true>(ab, stride, 0, x, p0, p1, sp, cnt);
-    for (i = U; i + U <= k; i += U) sturm_block<U, E, false>(ab, stride, i, x, p0, p1, sp, cnt);
+    sturm_block<U, E, true, RES>(ab, stride, 0, x, p0, p1, sp, cnt);
+    for (i = U; i + U <= k; i += U) sturm_block<U, E, false, RES>(ab, stride, i, x, p0, p1, sp, cnt);
   }
   const int r = k - i;
   if (U > 8 && r >= 12) {
-    sturm_block<(U > 8 ? 12 : 4), E, false>(ab, stride, i, x, p0, p1, sp, cnt);
+    sturm_block<(U > 8 ? 12 : 4), E, false, RES>(ab, stride, i, x, p0, p1, sp, cnt);
     i += 12;
   } else if (U > 8 && r >= 8) {
-    sturm_block<8, E, false>(ab, stride, i, x, p0, p1, sp, cnt);
+    sturm_block<8, E, false, RES>(ab, stride, i, x, p0, p1, sp, cnt);
     i += 8;
   } else if (r >= 4) {
-    sturm_block<4, E, false>(ab, stride, i, x, p0, p1, sp, cnt);
+    sturm_block<4, E, false, RES>(ab, stride, i, x, p0, p1, sp, cnt);
     i += 4;
   }
   for (; i < k; ++i) {
     const double2 t = ab[(size_t)i * stride];
 #pragma unroll
     for (int e = 0; e < E; ++e) {
+      if (i > 0 && (i & (RES - 1)) == 0) sturm_rescale(p0[e], p1[e]);
       const double p2 = fma(t.x - x[e], p1[e], i > 0 ? -t.y * p0[e] : 0.0);
       const unsigned s2 = (unsigned)__double2hiint(p2) >> 31;
       cnt[e] += (int)(s2 ^ sp[e]);
@@ -137,17 +141,19 @@ __device__ __forceinline__ void sturm_counts(const double2* __restrict__ ab, int
   }
 }
 
-template <int U>
+template <int U, int RES = 16>
 __device__ __forceinline__ int sturm_count_strided(const double2* __restrict__ ab, int stride, int k,
                                                    double x) {
   const double xs[1] = {x};
   int cnt[1];
-  sturm_counts<U, 1>(ab, stride, k, xs, cnt);
+  sturm_counts<U, 1, RES>(ab, stride, k, xs, cnt);
   return cnt[0];
 }
 
+// T of any length k (the engines for k > 128 do not fill it up), rescaled every
+// 8 rows: a few rounds a set, so the wider range costs nothing that shows.
 __device__ __forceinline__ int sturm_count(const double2* __restrict__ ab, int k, double x) {
-  return sturm_count_strided<8>(ab, 1, k, x);
+  return sturm_count_strided<8, 8>(ab, 1, k, x);
 }
 
 // The same count a row at a time, in few registers: for the kernels of many
