@@ -54,6 +54,7 @@ extern "C" {
 #define PL_SET_NONFINITE 2  /* NaN/Inf in the submatrix or the recurrence    */
 #define PL_SET_BAD_INDEX 4  /* an index outside [0, n)                       */
 #define PL_SET_BAD_K 8      /* k outside [1, PL_KMAX]                         */
+#define PL_SET_TIMEDOUT 16  /* a bounded wait inside its kernel gave up (k > 128) */
 
 /* ---- forms -------------------------------------------------------------- */
 #define PL_FORM_BATCHED 0   /* persistent, binned by k, register-resident    */
@@ -80,7 +81,9 @@ int pl_last_cuda_error(void);              /* cudaError_t of the last PL_ECUDA *
  *   lmin, lmax, delta (FP64, nsets), err (int32, nsets): each nullable
  *   eig     nullable; all k eigenvalues ascending at the set's index offset
  *   det     nullable; product of the eigenvalues (FP64, nsets)
- * Per-set problems are reported in err[], not as a failed call.
+ * Per-set problems are reported in err[], not as a failed call.  (k > 128: a
+ * set's CTAs wait for one another for 2 s at most; sets that time out are NaN
+ * with PL_SET_TIMEDOUT, and pl_solve_host returns PL_ETIMEDOUT.)
  */
 int pl_solve(const float *A, int n, long long lda, const int *idx, const long long *offsets,
              long long nsets, int k, int form, double *lmin, double *lmax, double *delta,

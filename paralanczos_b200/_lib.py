@@ -12,7 +12,7 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(PKG, "libparalanczos_b200.so")
 
 PL_OK, PL_EINVAL, PL_ECUDA, PL_ENOMEM, PL_ENOTSUP, PL_ETIMEDOUT, PL_EBUSY = range(7)
-PL_SET_BREAKDOWN, PL_SET_NONFINITE, PL_SET_BAD_INDEX, PL_SET_BAD_K = 1, 2, 4, 8
+PL_SET_BREAKDOWN, PL_SET_NONFINITE, PL_SET_BAD_INDEX, PL_SET_BAD_K, PL_SET_TIMEDOUT = 1, 2, 4, 8, 16
 PL_FORM_BATCHED, PL_FORM_PLAIN = 0, 1
 PL_KMAX = 512
 

@@ -298,7 +298,12 @@ cudaError_t launch_cluster(const MatrixF32& M, const SetSource& src, const SetOu
   if (verbosity() >= 2)
     fprintf(stderr, "paralanczos: cluster KB=%d CS=%d NTC=%d: %lld clusters (max resident %d), %zu B smem/CTA\n",
             KB, CS, NTC, ncl, maxcl, dsm);
-  kern<<<(unsigned)(ncl * CS), NTC, dsm, st>>>(M, src, out);
+  // PL_CLUSTER_TEST_HOLD=1 or 2 (tests of the timeout path only): the last CTA of
+  // every cluster holds its sends back until its peers' waits have run out, or
+  // gives up behind its first set's last step; the sets come back as timed out.
+  const char* h = CS > 1 ? getenv("PL_CLUSTER_TEST_HOLD") : nullptr;
+  const int hold = h && (h[0] == '1' || h[0] == '2') ? h[0] - '0' : 0;
+  kern<<<(unsigned)(ncl * CS), NTC, dsm, st>>>(M, src, out, hold);
   return cudaGetLastError();
 }
 
@@ -521,6 +526,9 @@ struct DevState {
     cudaGraphExec_t exec;
   };
   std::unordered_map<std::string, GraphEntry> graphs;
+  // Host-buffer calls: 1 once a set of the call timed out (pinned host memory,
+  // written by the kernels).
+  int* timed_out = nullptr;
 };
 
 DevState g_state[64];
@@ -673,9 +681,10 @@ int solve_csr(const MatrixF32& M, const int* idx, const long long* offsets, long
   rc = ensure(d.large, qtotal > 0 ? qtotal : 256);
   if (rc) return rc;
   char keybuf[512];
-  int kl = snprintf(keybuf, sizeof keybuf, "%p|%d|%lld|%p|%p|%lld|%d|%p|%p|%p|%p|%p|%p|", (const void*)M.A, M.n,
+  int kl = snprintf(keybuf, sizeof keybuf, "%p|%d|%lld|%p|%p|%lld|%d|%p|%p|%p|%p|%p|%p|%p|", (const void*)M.A, M.n,
                     M.lda, (const void*)idx, (const void*)offsets, nsets, form, (void*)out.lmin,
-                    (void*)out.lmax, (void*)out.delta, (void*)out.err, (void*)out.eig, (void*)out.det);
+                    (void*)out.lmax, (void*)out.delta, (void*)out.err, (void*)out.eig, (void*)out.det,
+                    (void*)out.status);
   for (int b = 0; b < kNumBins && kl > 0 && kl < (int)sizeof keybuf - 4; ++b)
     kl += snprintf(keybuf + kl, sizeof keybuf - (size_t)kl, "%d,", g_variant[b]);
   const std::string key(keybuf);
@@ -1060,6 +1069,9 @@ int pl_solve_host(const float* A, int n, long long lda, const int* idx, const lo
   if (idx_src == dI) PL_CU(cudaMemcpyAsync(dI, idx, sizeof(int) * total, cudaMemcpyHostToDevice, st));
   if (dO) PL_CU(cudaMemcpyAsync(dO, offsets, sizeof(long long) * (nsets + 1), cudaMemcpyHostToDevice, st));
   SetOutputs out{dmin, dmax, ddel, derr, deig, ddet};
+  if (!d.timed_out) PL_CU(cudaHostAlloc((void**)&d.timed_out, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
+  *d.timed_out = 0;
+  out.status = d.timed_out;  // (unified addressing: the same pointer on the device)
   rc = solve_dev(dA, n, lda, idx_src, dO, nsets, k, form, out, st);
   if (rc) return rc;
   if (lmin) PL_CU(cudaMemcpyAsync(lmin, dmin, sizeof(double) * nsets, cudaMemcpyDeviceToHost, st));
@@ -1069,7 +1081,7 @@ int pl_solve_host(const float* A, int n, long long lda, const int* idx, const lo
   if (err) PL_CU(cudaMemcpyAsync(err, derr, sizeof(int) * nsets, cudaMemcpyDeviceToHost, st));
   if (eig) PL_CU(cudaMemcpyAsync(eig, deig, sizeof(double) * total, cudaMemcpyDeviceToHost, st));
   PL_CU(cudaStreamSynchronize(st));
-  return PL_OK;
+  return *(volatile int*)d.timed_out ? PL_ETIMEDOUT : PL_OK;
 }
 
 int pl_gather_blocks(const float* A, int n, long long lda, const int* idx, long long nsets, int k,
@@ -1210,6 +1222,8 @@ int pl_release(void) {
     s->p = nullptr;
     s->bytes = 0;
   }
+  if (d.timed_out) cudaFreeHost(d.timed_out);
+  d.timed_out = nullptr;
   d.mc.valid = false;
   gram_release();
   return PL_OK;

@@ -85,7 +85,8 @@ struct __align__(16) ClusterSmem {
   double red[NTC / 32];          // warp partials inside the CTA (breakdown argmax)
   unsigned long long key[CS];    // breakdown argmax exchange
   unsigned long long bar[2];     // mbarriers of the y and the w exchange
-  int abort;                     // a bounded wait gave up
+  int abort;                     // a bounded wait gave up, here or in a peer
+  long long lost;                // the item it was on
 };
 
 // What one exchange delivers into every CTA: KB rows and the warps' partials.
@@ -182,8 +183,15 @@ enum ClusterResult { CLUSTER_DONE, CLUSTER_RESTARTED, CLUSTER_BROKE, CLUSTER_ABO
 //   DONE       its outputs are written
 //   RESTARTED  the same, and it had a breakdown (RESTART)
 //   BROKE      it had a breakdown, nothing is written (!RESTART)
-//   ABORT      a bounded wait gave up: it is reported as failed, and the kernel
-//              must end
+//   ABORT      a bounded wait gave up somewhere in the cluster: nothing is
+//              written, and every CTA of the cluster must end
+// A wait that gives up is a warp's answer first, then the CTA's (a vote in
+// every step, and at the end of the steps), then the cluster's: no CTA passes
+// the barrier at the end of its steps before every other one is there, and
+// behind it all know whether one of them gave up, so they leave together and no
+// CTA writes into one that has left.  hold (tests): 1, the last CTA stays out of
+// the steps until its peers' waits have run out; 2, it gives up behind the last
+// one, when its peers have all they need.
 // RESTART: with the breakdown restart.  P then has to outlive the step loop,
 // which costs the loop 80 to 400 bytes of spills at 168 and 255 registers
 // wherever the restart stands (k = 512 1.04 -> 1.25 ms a set, k = 384 0.86 ->
@@ -196,7 +204,7 @@ __device__ __forceinline__ ClusterResult cluster_solve_set(const MatrixF32& M, c
                                                   int k, long long set, const SetOutputs& out,
                                                   ClusterSmem<KB, CS, NTC>& sm,
                                                   cg::cluster_group& cl, int rank, uint32_t& ph,
-                                                  uint32_t ta) {
+                                                  uint32_t ta, int hold) {
   using C = CfgC<KB, CS, NTC, RPT>;
   constexpr int R = C::R, RS = C::RS, TPR = C::TPR, CPT = C::CPT, NCH = C::NCH;
   constexpr int NPART = ClusterSmem<KB, CS, NTC>::NPART;
@@ -235,12 +243,16 @@ __device__ __forceinline__ ClusterResult cluster_solve_set(const MatrixF32& M, c
       if (lane < CS) st_async(peer_addr(smem_u32(pd), lane), x, peer_addr(bar, lane));
     }
   };
-  bool ok = true;
-  auto arrived = [&](uint32_t bar) {
+  // Waits for an exchange; false: the thread gave up.  The warp's lanes are
+  // together again afterwards, for the matrix products that follow.
+  auto arrived = [&](uint32_t bar) -> bool {
     if constexpr (CS == 1) {
       __syncthreads();
+      return true;
     } else {
-      if (ok) ok = mbar_wait(bar, ph, (volatile int*)&sm.abort, nullptr);
+      const bool got = mbar_wait(bar, ph, (volatile int*)&sm.abort, nullptr);
+      __syncwarp();
+      return got;
     }
   };
 
@@ -360,9 +372,13 @@ __device__ __forceinline__ ClusterResult cluster_solve_set(const MatrixF32& M, c
   int status = 0;
   int cur = 0, prv = 1, nxt = 2;
   __syncthreads();
+  TmemBuf<NB> buf[2];
+  if (CS > 1 && hold == 1 && rank == CS - 1) {
+    for (const unsigned long long t0 = globaltimer(); globaltimer() - t0 < kWaitNs + kWaitNs / 4;) __nanosleep(10000);
+    goto lost;
+  }
   // Steps run in segments: a breakdown leaves the step loop, restarts the
   // recurrence from P in shared memory and enters the loop again.
-  TmemBuf<NB> buf[2];
   for (int j = 0;; ++j) {
     float2 Pr[RPT][CPT / 2];
 #pragma unroll
@@ -431,7 +447,7 @@ __device__ __forceinline__ ClusterResult cluster_solve_set(const MatrixF32& M, c
       ve[e] = c < KB ? sc * sm.vb[cur][c] : 0.f;
       we[e] = c < KB ? scp * sm.vb[prv][c] : 0.f;
     }
-    arrived(ybar);
+    const bool got_y = arrived(ybar);
 #pragma unroll
     for (int e = 0; e < NE; ++e) we[e] = fmaf(-bprev, we[e], t + e * NTC < KB ? sm.yb[t + e * NTC] : 0.f);
     const double alpha = part_sum<NPART>(sm.part[0]);
@@ -442,7 +458,7 @@ __device__ __forceinline__ ClusterResult cluster_solve_set(const MatrixF32& M, c
     if constexpr (CS == 1) {
       __syncthreads();
     } else {
-      if (__syncthreads_or(!ok)) goto done;
+      if (__syncthreads_or(!got_y)) goto failed;
     }
 
     // w = P w~ over the owned row slices
@@ -468,11 +484,13 @@ __device__ __forceinline__ ClusterResult cluster_solve_set(const MatrixF32& M, c
     publish_row(sm.vb[nxt], wo, wbar);
     publish_partial(1, warp_sum(lead ? (double)wo * (double)wo : 0.0), wbar);
     buf[0].load(ta, 0);  // the next pass's first buffer
-    arrived(wbar);
+    const bool got_w = arrived(wbar);
 #pragma unroll
     for (int q = 0; q < RPT; ++q) v[q] = sm.vb[nxt][r[q]];
-    // (after a wait that gave up, the next barrier ends the loop)
-    const double b2v = ok ? part_sum<NPART>(sm.part[1]) : 1.0;
+    const double b2v = part_sum<NPART>(sm.part[1]);
+    // (such a warp votes at once, the CTA's others at their next vote; asked here,
+    // behind the sum, it is free: before it, 1.02 times the step at k = 512)
+    if (CS > 1 && __any_sync(0xffffffffu, !got_w)) goto lost;
     ph ^= 1u;
     if (t == 0 && rank == 0) {
       sm.ab[j].x = alpha;
@@ -480,9 +498,9 @@ __device__ __forceinline__ ClusterResult cluster_solve_set(const MatrixF32& M, c
     }
     if (!isfinite(alpha) || !isfinite(b2v)) {
       status |= SET_NONFINITE;
-      goto done;
+      goto steps_done;
     }
-    if (j + 1 == k) goto done;
+    if (j + 1 == k) goto steps_done;
     if (!(b2v > tau2)) break;
     const float bf = sqrtf((float)b2v);
     scp = sc;
@@ -497,7 +515,14 @@ __device__ __forceinline__ ClusterResult cluster_solve_set(const MatrixF32& M, c
     nxt = old_prv;
   }
     buf[0].ready();  // no load outlives the segment
-    if constexpr (!RESTART) return CLUSTER_BROKE;
+    if constexpr (!RESTART) {
+      if constexpr (CS > 1) {
+        if (__syncthreads_or(0)) goto failed;
+        set_sync<CS>(cl);
+        if (sm.abort) goto leave;
+      }
+      return CLUSTER_BROKE;
+    }
     // Breakdown: restart from the column of P with the largest diagonal
     // (cluster-wide argmax, ties to the smaller row), published into vb[nxt].
     status |= SET_BREAKDOWN;
@@ -509,7 +534,13 @@ __device__ __forceinline__ ClusterResult cluster_solve_set(const MatrixF32& M, c
         p2[0] = Pr[q][2 * ch];
         p2[1] = Pr[q][2 * ch + 1];
       }
-    __syncthreads();
+    if constexpr (CS > 1) {
+      if (__syncthreads_or(0)) goto failed;
+      set_sync<CS>(cl);
+      if (sm.abort) goto leave;
+    } else {
+      __syncthreads();
+    }
     unsigned long long kk = 0ull;
     for (int e = t; e < R && rank * R + e < k; e += NTC) {
       const int row = rank * R + e;
@@ -558,16 +589,15 @@ __device__ __forceinline__ ClusterResult cluster_solve_set(const MatrixF32& M, c
     cur = nxt;
     nxt = old_prv;
   }
-done:
+steps_done:
   buf[0].ready();  // no load outlives the set
   if constexpr (CS > 1) {
-    if (__syncthreads_or(!ok)) {
-      if (rank == 0 && t == 0) write_failed(out, set, 0, 0, SET_NONFINITE);
-      set_sync<CS>(cl);  // every peer's waits give up too; none of its copies is in flight
-      return CLUSTER_ABORT;
-    }
+    if (__syncthreads_or(hold == 2 && rank == CS - 1)) goto failed;
   }
   set_sync<CS>(cl);  // every rank done with the step loop before T is read
+  if constexpr (CS > 1) {
+    if (sm.abort) goto leave;
+  }
 
   // ---- extremes on rank 0: warp 0 lambda_min, warp 1 lambda_max, 33-way -----
   if (rank == 0) {
@@ -602,6 +632,17 @@ done:
   }
   set_sync<CS>(cl);  // rank 0's reads of T precede the next set's writes
   return (status & SET_BREAKDOWN) ? CLUSTER_RESTARTED : CLUSTER_DONE;
+
+lost:  // this warp: its vote
+  __syncthreads_or(1);
+failed:  // this CTA
+  if (t < CS) *(volatile int*)&cl.map_shared_rank(&sm, (unsigned)t)->abort = 1;
+  set_sync<CS>(cl);
+leave:  // every CTA of the cluster
+  // (what a peer sent and no wait here counted has long arrived after 1 ms)
+  for (const unsigned long long t0 = globaltimer(); globaltimer() - t0 < 1000000ull;) __nanosleep(1000);
+  set_sync<CS>(cl);
+  return CLUSTER_ABORT;
 }
 
 }  // namespace pl

@@ -14,6 +14,7 @@ enum SetStatus : int {
   SET_NONFINITE = 2,     // NaN/Inf met in the submatrix or the recurrence
   SET_BAD_INDEX = 4,     // an index of the set is outside [0, n)
   SET_BAD_K = 8,         // the set's k is outside the kernel's supported range
+  SET_TIMEDOUT = 16,     // a bounded wait between the CTAs of its cluster gave up
 };
 
 constexpr float kEps32 = 1.1920929e-7f;
@@ -36,6 +37,7 @@ struct SetOutputs {
   int* err;       // SetStatus bits (nullable)
   double* eig;    // all k eigenvalues ascending at the set's index offset (nullable)
   double* det;    // product of eigenvalues (nullable)
+  int* status = nullptr;  // 1 if a set timed out (nullable; host memory mapped into the device)
 };
 
 // One device-resident matrix of a table (serving: sets of one launch may

@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(256, 1)
 // ---------------------------------------------------------------------------
 template <int KB, int CS, int NTC, int RPT, int NB>
 __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NTC, 1)
-    k_cluster_solve(MatrixF32 M, SetSource src, SetOutputs out) {
+    k_cluster_solve(MatrixF32 M, SetSource src, SetOutputs out, int hold) {
   extern __shared__ __align__(16) float dsm[];
   ClusterSmem<KB, CS, NTC>& sm = *reinterpret_cast<ClusterSmem<KB, CS, NTC>*>(dsm);
   cg::cluster_group cl = cg::this_cluster();
@@ -303,7 +303,6 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NTC, 1)
   uint32_t ph = 0;
   TmemA<KB / CS * KB / NTC, NTC, NB> am;
   am.begin();
-  ClusterResult res = CLUSTER_DONE;
   bool likely_breaks = false;
   const long long nitems = item_count(src);
   const int pbase = src.perm_start ? *src.perm_start : 0;
@@ -315,22 +314,39 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NTC, 1)
       if (rank == 0 && threadIdx.x == 0) write_failed(out, set, off, 0, SET_BAD_K);
       continue;
     }
+    ClusterResult res = CLUSTER_DONE;
     // one CTA: the loop fits its registers with the restart (0.30 ms a set
     // either way at k = 192, and a breakdown costs no second solve).  A set after
     // one that broke down is likely to break down too.
     if constexpr (CS > 1) {
       if (!likely_breaks) {
-        res = cluster_solve_set<KB, CS, NTC, RPT, NB, false>(M, src.idx + off, k, set, out, sm, cl, rank, ph, am.ta);
+        res = cluster_solve_set<KB, CS, NTC, RPT, NB, false>(M, src.idx + off, k, set, out, sm, cl, rank, ph, am.ta,
+                                                             hold);
         likely_breaks = res == CLUSTER_BROKE;
       }
     }
     if (CS == 1 || likely_breaks) {
-      res = cluster_solve_set<KB, CS, NTC, RPT, NB, true>(M, src.idx + off, k, set, out, sm, cl, rank, ph, am.ta);
+      res = cluster_solve_set<KB, CS, NTC, RPT, NB, true>(M, src.idx + off, k, set, out, sm, cl, rank, ph, am.ta,
+                                                          hold);
       likely_breaks = res == CLUSTER_RESTARTED;
     }
-    if (res == CLUSTER_ABORT) break;
+    if (CS > 1 && res == CLUSTER_ABORT) {
+      if (threadIdx.x == 0) sm.lost = it;
+      break;
+    }
   }
   am.end();
+  // A cluster that timed out: its set and all that it had still to solve.
+  if (CS > 1 && rank == 0 && threadIdx.x == 0 && sm.abort) {
+    const long long end = item_count(src);  // (read again, as is all else: held through the sets it spills)
+    for (long long it = sm.lost; it < end; it += gridDim.x / CS) {
+      long long set, off;
+      int k;
+      set_span(src, it, src.perm_start ? *src.perm_start : 0, set, off, k);
+      write_failed(out, set, off, 0, k < 1 || k > KB ? SET_BAD_K : SET_TIMEDOUT);
+    }
+    if (out.status) *(volatile int*)out.status = 1;
+  }
 }
 
 // ---------------------------------------------------------------------------

@@ -45,7 +45,7 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
 
 // Bounded wait for the phase with the given parity.  false: gave up (timeout
 // here, or another role already aborted); the abort flag is then set and, if
-// status is given, *status = 1.
+// status is given, *status = 1.  The answer is the thread's own.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort,
                                           int* status) {
   if (mbar_try(bar, parity)) return true;

@@ -109,6 +109,7 @@ struct TmemA {
   }
   __device__ __forceinline__ void end() {
     if constexpr (NB > 0) {
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");  // (a set given up leaves a load behind)
       __syncthreads();
       if (threadIdx.x < 32) tmem_free(base, kAlloc);
     }
