@@ -342,6 +342,8 @@ struct Variant {
   // (extremes mode) each group reads its next set's indices one set ahead,
   // so their latency is hidden behind a whole set's Lanczos steps
   bool indices_ahead;
+  // (all eigenvalues) the kernel that calls of few sets run: the same bits
+  LaunchFn few_all;
 };
 
 #define REG(KB, RPT, TPR, CTA, MINB)                                                          \
@@ -370,12 +372,14 @@ struct Variant {
         true                                                                                     \
   }
 // the same with A_S in tensor memory (NB float4 per load); all eigenvalues at up
-// to 255 registers (the bisection holds 16 rows of T and their minors twice)
+// to 255 registers (the bisection holds 16 rows of T and their minors twice), calls
+// of few sets on the register engine, two warps per set
 #define SAPT(KB, RPT, CTA, REGS, NB)                                                         \
   Variant {                                                                                    \
     "tmemA ahead KB=" #KB " RPT=" #RPT " CTA=" #CTA " REGS=" #REGS " NB=" #NB,                 \
         {launch_sap<KB, RPT, CTA, REGS, NB>, launch_sap<KB, RPT, CTA, 255, NB, true>},          \
-        {scratch_sap<KB, RPT, CTA, REGS, NB>, scratch_none}, true                               \
+        {scratch_sap<KB, RPT, CTA, REGS, NB>, scratch_none}, true,                              \
+        launch_reg<KB, 1, 1, 128, 3, true>                                                      \
   }
 // two threads per row, RPT rows per thread, A_S in tensor memory (NB float4 per
 // load); all eigenvalues: one row per thread (the bin's other FP32 sums) with
@@ -466,21 +470,16 @@ const Variant& chosen_for(int b, bool all) {
   return v;
 }
 
-// The same for a call of nsets sets.  All eigenvalues at 48 < k <= 64 by the
-// tensor-memory kernel (8 sets an SM at once, one warp each): a few sets take
-// 6/5 of the time of the register kernel's (6 sets an SM, two warps each), so
-// that one runs where its waves are the cheaper ones (k = 64: 300 sets 112 -> 96
-// us, 2,400 391 -> 335; 4,800 665 -> 648; but 900, two waves against one, 146
-// against 191, and 10,000 1,201 against 1,281).  Neither needs scratch; their
-// FP32 sums are the same, their FP64 sums differ in the last bits.
-const Variant& variant_for(int b, bool all, long long nsets) {
-  const Variant& v = chosen_for(b, all);
-  if (kBinK[b] == 64 && all && g_variant[b] == 10 && nsets >= 0) {
-    const long long sms = device_sms();
-    const long long reg = (nsets + 6 * sms - 1) / (6 * sms), tmem = (nsets + 8 * sms - 1) / (8 * sms);
-    if (5 * reg <= 6 * tmem) return variants(b)[0];
-  }
-  return v;
+// All eigenvalues at 48 < k <= 64 by the tensor-memory kernel (8 sets an SM at
+// once, one warp each): a few sets take 6/5 of the time of the register kernel's
+// (6 sets an SM, two warps each), so that one runs where its waves are the cheaper
+// ones (k = 64: 300 sets 112 -> 96 us, 2,400 391 -> 335; 4,800 665 -> 648; but
+// 900, two waves against one, 146 against 191, and 10,000 1,201 against 1,281).
+// Neither needs scratch, and their results are the same, bit for bit.
+LaunchFn few_all_fn(const Variant& v, long long nsets) {
+  const long long sms = device_sms();
+  const long long reg = (nsets + 6 * sms - 1) / (6 * sms), tmem = (nsets + 8 * sms - 1) / (8 * sms);
+  return v.few_all && 5 * reg <= 6 * tmem ? v.few_all : nullptr;
 }
 
 // Plain form kernels by k bin (k <= 128).
@@ -587,9 +586,9 @@ int solve_uniform(const MatrixF32& M, const int* idx, long long nsets, int k, in
     PL_CU(plain_fn(k, all)(M, src, out, nsets, nullptr, st, false));
     return PL_OK;
   }
-  int b = bin_of_k(k);
+  const int b = bin_of_k(k);
   if (b < 0) return PL_ENOTSUP;
-  const Variant& v = variant_for(b, all, nsets);
+  const Variant& v = chosen_for(b, all);
   void* scratch = nullptr;
   const size_t need = v.scratch[all ? 1 : 0]();
   if (need) {
@@ -597,7 +596,20 @@ int solve_uniform(const MatrixF32& M, const int* idx, long long nsets, int k, in
     if (rc) return rc;
     scratch = state().large.p;
   }
-  PL_CU(v.fn[all ? 1 : 0](M, src, out, nsets, scratch, st, false));
+  LaunchFn fn = v.fn[all ? 1 : 0];
+  if (all && v.few_all) {
+    // (both are loaded by the first call: a later one of the other size may be captured)
+    static bool loaded[64] = {};
+    int dev = 0;
+    PL_CU(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || !loaded[dev]) {
+      PL_CU(fn(M, src, out, 0, nullptr, st, true));
+      PL_CU(v.few_all(M, src, out, 0, nullptr, st, true));
+      if (dev >= 0 && dev < 64) loaded[dev] = true;
+    }
+    if (LaunchFn few = few_all_fn(v, nsets)) fn = few;
+  }
+  PL_CU(fn(M, src, out, nsets, scratch, st, false));
   return PL_OK;
 }
 
@@ -613,10 +625,10 @@ size_t binned_qscratch(int form, bool all, size_t off[kNumBins]) {
   return total;
 }
 
-void binned_fns(int form, bool all, long long nsets, LaunchFn fns[kNumBins]) {
+void binned_fns(int form, bool all, LaunchFn fns[kNumBins]) {
   for (int b = 0; b < kNumBins; ++b)
     fns[b] = (form == PL_FORM_PLAIN && kBinK[b] <= 128) ? plain_fn(kBinK[b], all)
-                                                        : variant_for(b, all, nsets).fn[all ? 1 : 0];
+                                                        : chosen_for(b, all).fn[all ? 1 : 0];
 }
 
 // The binned sequence on stream cs: count sets per k bin, scan, scatter the
@@ -691,7 +703,7 @@ int solve_csr(const MatrixF32& M, const int* idx, const long long* offsets, long
   auto it = d.graphs.find(key);
   if (it == d.graphs.end()) {
     LaunchFn fns[kNumBins];
-    binned_fns(form, all, nsets, fns);
+    binned_fns(form, all, fns);
     // load every kernel before the capture: nothing that may load a module
     // or set a function attribute runs while the stream is capturing
     for (int b = 0; b < kNumBins; ++b) PL_CU(fns[b](M, SetSource{}, out, 0, nullptr, d.side[b], true));
@@ -772,7 +784,7 @@ size_t api_binned_scratch(long long nsets, int form, bool all) {
 }
 int api_prepare_binned(int form, bool all) {
   LaunchFn fns[kNumBins];
-  binned_fns(form, all, -1, fns);
+  binned_fns(form, all, fns);
   SetOutputs out{};
   for (int b = 0; b < kNumBins; ++b) PL_CU(fns[b](MatrixF32{}, SetSource{}, out, 0, nullptr, 0, true));
   return PL_OK;
@@ -786,7 +798,7 @@ int api_launch_binned(const MatrixF32& M, const int* idx, const long long* offse
   size_t qoff[kNumBins];
   binned_qscratch(form, all, qoff);
   LaunchFn fns[kNumBins];
-  binned_fns(form, all, nsets_dev ? -1 : nsets, fns);
+  binned_fns(form, all, fns);
   char* base = (char*)scratch;
   int* hdr = (int*)base;
   char* q = base + align256(sizeof(int) * (48 + (size_t)nsets));

@@ -48,6 +48,7 @@ struct __align__(16) GroupSmem {
   int idx[KB];          // the set's indices
   double2 ab[KB];       // T: ab[i] = {alpha_i, beta_i^2}, beta_i couples rows i-1, i
   double red[6][NW];    // cross-warp partials (slots 4/5: lambda_min/max hand-off)
+  double row[2][KB == 64 && NW == 2 ? 64 : 1];  // one value per row (SAME_SUMS)
 };
 
 template <int NT>
@@ -201,6 +202,11 @@ __device__ __forceinline__ int solve_set(const MatrixF32& M, const int* __restri
                                           GroupSmem<KB, Cfg<KB, RPT, TPR>::NW>& sm,
                                           const Grp<Cfg<KB, RPT, TPR>::NT>& g) {
   using C = Cfg<KB, RPT, TPR>;
+  // All eigenvalues at 48 < k <= 64: calls of few sets run here, with two warps
+  // per set, calls of many on solve_set_sa with one, and a set's results do not
+  // depend on its call.  So both read the same triangle of A and take every FP64
+  // sum and product in the same order.
+  constexpr bool SAME_SUMS = ALL && KB == 64 && RPT == 1 && TPR == 1;
   constexpr int NT = C::NT;
   constexpr int NW = C::NW;
   constexpr int CPT = C::CPT;
@@ -242,9 +248,17 @@ __device__ __forceinline__ int solve_set(const MatrixF32& M, const int* __restri
 #pragma unroll
     for (int cc = 0; cc < CPT; cc += 2) {
       const int c = c0 + cc;
-      const float a0 = (rv & (c < k)) ? __ldg(arow + sm.idx[c]) : 0.f;
-      const float a1 = (rv & (c + 1 < k)) ? __ldg(arow + sm.idx[c + 1]) : 0.f;
-      Ar[q][cc / 2] = make_float2(a0, a1);
+      if constexpr (SAME_SUMS) {  // the upper triangle
+        const float* __restrict__ p0 =
+            c >= r ? arow + sm.idx[c] : SM.A + (size_t)sm.idx[c] * (size_t)SM.lda + sm.idx[r];
+        const float* __restrict__ p1 =
+            c + 1 >= r ? arow + sm.idx[c + 1] : SM.A + (size_t)sm.idx[c + 1] * (size_t)SM.lda + sm.idx[r];
+        Ar[q][cc / 2] = make_float2((rv & (c < k)) ? __ldg(p0) : 0.f, (rv & (c + 1 < k)) ? __ldg(p1) : 0.f);
+      } else {
+        const float a0 = (rv & (c < k)) ? __ldg(arow + sm.idx[c]) : 0.f;
+        const float a1 = (rv & (c + 1 < k)) ? __ldg(arow + sm.idx[c + 1]) : 0.f;
+        Ar[q][cc / 2] = make_float2(a0, a1);
+      }
     }
   }
   // (after all the loads are issued: an FP64 use of each value behind its load
@@ -258,10 +272,32 @@ __device__ __forceinline__ int solve_set(const MatrixF32& M, const int* __restri
       const int c = c0 + cc;
       const float2 e = Ar[q][cc / 2];
       Pr[q][cc / 2] = make_float2((rv && c == r) ? 1.f : 0.f, (rv && c + 1 == r) ? 1.f : 0.f);
-      fro += (double)e.x * (double)e.x + (double)e.y * (double)e.y;
+      if constexpr (!SAME_SUMS) fro += (double)e.x * (double)e.x + (double)e.y * (double)e.y;
     }
   }
-  const double fro2 = group_sum<NT, NW>(fro, g, sm.red[2]);
+  double fro2;
+  if constexpr (SAME_SUMS) {
+    // a lane there adds the upper elements of row p, then those of row 63 - p: warp
+    // 0 adds its rows, warp 1 goes on from there
+#pragma unroll 1
+    for (int w = 0; w < 2; ++w) {
+      if (g.wig == w) {
+        if (w == 1) fro = sm.row[1][63 - t];
+#pragma unroll
+        for (int c = 0; c < KB; ++c) {
+          const double x = c & 1 ? Ar[0][c / 2].y : Ar[0][c / 2].x;
+          if (c == t) sm.row[0][t] = x * x;
+          if (c > t) fro += x * x;
+        }
+        sm.row[1][t] = fro;
+      }
+      g.sync();
+    }
+    const int p = t & 31;
+    fro2 = warp_sum((sm.row[0][p] + sm.row[0][63 - p]) + 2.0 * sm.row[1][63 - p]);
+  } else {
+    fro2 = group_sum<NT, NW>(fro, g, sm.red[2]);
+  }
   const double tau = 32.0 * (double)kEps32 * sqrt(fro2);
 
   // ---- Lanczos with projector reorthogonalisation ----------------------------

@@ -148,6 +148,19 @@ __device__ __forceinline__ int solve_set_sa(const MatrixF32& M, const int* __res
   constexpr int NT = C::NT;
   constexpr int NW = C::NW;
   constexpr int NCH = C::NCH;
+  // (as in solve_set, whose two warps hold one row per thread: the sums of rows
+  // t and of rows t + 32 one by one, then added)
+  constexpr bool SAME_SUMS = ALL && KB == 64 && RPT == 2;
+  const auto row_sum = [&](double (&x)[RPT], double* red) -> double {
+    if constexpr (SAME_SUMS) {
+      return warp_sum(x[0]) + warp_sum(x[1]);
+    } else {
+      double s = 0.0;
+#pragma unroll
+      for (int q = 0; q < RPT; ++q) s += x[q];
+      return group_sum<NT, NW>(s, g, red);
+    }
+  };
   const int t = g.t;
   if constexpr (PF) {
     static_assert(RPT <= 2, "the prefetch follows the triangle gather");
@@ -202,11 +215,11 @@ __device__ __forceinline__ int solve_set_sa(const MatrixF32& M, const int* __res
       const int r0 = p, r1 = KB - 1 - p;
       const float* __restrict__ row0 = SM.A + (size_t)sm.idx[r0] * (size_t)SM.lda;
       const float* __restrict__ row1 = SM.A + (size_t)sm.idx[r1] * (size_t)SM.lda;
+      double fa = 0.0, fb = 0.0;  // diagonal, upper triangle
       if (PF && have) {
         // from the stage, U elements at a time: read ahead of their stores, which
         // could alias the next reads (one at a time took 230 cycles an element)
         constexpr int U = 13;
-        double fa = 0.0, fb = 0.0;  // diagonal, upper triangle
         for (int ii = 0; ii < PER; ii += U) {
           float e[U];
 #pragma unroll
@@ -226,7 +239,6 @@ __device__ __forceinline__ int solve_set_sa(const MatrixF32& M, const int* __res
             }
           }
         }
-        fro = fa + 2.0 * fb;
       } else {
 #pragma unroll 8
         for (int ii = 0; ii < PER; ++ii) {
@@ -238,11 +250,12 @@ __device__ __forceinline__ int solve_set_sa(const MatrixF32& M, const int* __res
           float e = 0.f;
           if (r < k && c < k) e = __ldg((first ? row0 : row1) + sm.idx[c]);
           const double e2 = (double)e * (double)e;
-          fro += (c == r) ? e2 : 2.0 * e2;
+          if (c == r) fa += e2; else fb += e2;
           Af[sa_at<NT, NCH>(r, c)] = e;
           if (c != r) Af[sa_at<NT, NCH>(c, r)] = e;
         }
       }
+      fro = fa + 2.0 * fb;
 #pragma unroll
       for (int q = 0; q < RPT; ++q) {
         const int r = t + q * NT;
@@ -360,13 +373,13 @@ __device__ __forceinline__ int solve_set_sa(const MatrixF32& M, const int* __res
       }
     }
     float yy[RPT];
-    double ap = 0.0;
+    double ap[RPT];  // (products of two floats: exact)
 #pragma unroll
     for (int q = 0; q < RPT; ++q) {
       yy[q] = ((ya[q].x + ya[q].y) + (yb[q].x + yb[q].y)) * sc;
-      ap = fma((double)v[q], (double)yy[q], ap);
+      ap[q] = (double)v[q] * (double)yy[q];
     }
-    const double alpha = group_sum<NT, NW>(ap, g, sm.red[0]);
+    const double alpha = row_sum(ap, sm.red[0]);
     const float af = (float)alpha;
 
     float wt[RPT];
@@ -395,15 +408,15 @@ __device__ __forceinline__ int solve_set_sa(const MatrixF32& M, const int* __res
       }
     }
     float ww[RPT];
-    double bp = 0.0;
+    double bp[RPT];
 #pragma unroll
     for (int q = 0; q < RPT; ++q) {
       ww[q] = (wa[q].x + wa[q].y) + (wc[q].x + wc[q].y);
-      bp = fma((double)ww[q], (double)ww[q], bp);
+      bp[q] = (double)ww[q] * (double)ww[q];
       sm.vb[t + q * NT] = ww[q];  // published by the sync below
     }
     if constexpr (NB > 0) buf[0].load(ta, 0);  // the next pass's first buffer
-    const double b2v = group_sum<NT, NW>(bp, g, sm.red[1]);
+    const double b2v = row_sum(bp, sm.red[1]);
     if constexpr (NW == 1) g.sync();
     if (t == 0) {
       sm.ab[j].x = alpha;
@@ -457,14 +470,14 @@ __device__ __forceinline__ int solve_set_sa(const MatrixF32& M, const int* __res
           }
         }
       g.sync();
-      double zp = 0.0;
+      double zp[RPT];
       float z[RPT];
 #pragma unroll
       for (int q = 0; q < RPT; ++q) {
         z[q] = sm.vb[t + q * NT];
-        zp += (double)z[q] * (double)z[q];
+        zp[q] = (double)z[q] * (double)z[q];
       }
-      const double zz = group_sum<NT, NW>(zp, g, sm.red[1]);
+      const double zz = row_sum(zp, sm.red[1]);
       if (t == 0) sm.ab[j + 1].y = 0x1p-600;  // decoupled block (see sturm_count)
       const float inv = 1.0f / sqrtf((float)zz);
       sc = inv;
@@ -506,7 +519,7 @@ __device__ __forceinline__ int solve_set_sa(const MatrixF32& M, const int* __res
   }
   {
     const int R = bisect_rounds(glo, ghi);
-    double prod = 1.0;
+    double prod = 1.0, prod1 = 1.0;  // (prod1: of eigenvalues t + 32, SAME_SUMS)
     // all of a thread's eigenvalues at once: their chains overlap
     constexpr int EV = (KB + NT - 1) / NT;
     for (int m0 = t; m0 < k; m0 += EV * NT) {
@@ -518,7 +531,7 @@ __device__ __forceinline__ int solve_set_sa(const MatrixF32& M, const int* __res
         if (m >= k) break;
         const double e = lam[v];
         if (out.eig) out.eig[off + m] = e;
-        prod *= e;
+        if (SAME_SUMS && v == 1) prod1 = e; else prod *= e;
         if (m == 0) {
           sm.red[4][0] = e;  // for delta, read after the sync below
           if (out.lmin) out.lmin[set] = e;
@@ -531,7 +544,11 @@ __device__ __forceinline__ int solve_set_sa(const MatrixF32& M, const int* __res
     }
     constexpr int W = NT < 32 ? NT : 32;
 #pragma unroll
-    for (int o = W / 2; o > 0; o >>= 1) prod *= __shfl_xor_sync(g.mask, prod, o);
+    for (int o = W / 2; o > 0; o >>= 1) {
+      prod *= __shfl_xor_sync(g.mask, prod, o);
+      if constexpr (SAME_SUMS) prod1 *= __shfl_xor_sync(g.mask, prod1, o);
+    }
+    if constexpr (SAME_SUMS) prod *= prod1;
     if constexpr (NW > 1) {
       if ((threadIdx.x & 31) == 0) sm.red[0][g.wig] = prod;
     }
