@@ -81,6 +81,9 @@ int pl_last_cuda_error(void);              /* cudaError_t of the last PL_ECUDA *
  *   lmin, lmax, delta (FP64, nsets), err (int32, nsets): each nullable
  *   eig     nullable; all k eigenvalues ascending at the set's index offset
  *   det     nullable; product of the eigenvalues (FP64, nsets)
+ * Calls on several streams share the library's scratch and run one after the
+ * other on the GPU where they need it.  Calls captured into a graph cannot wait
+ * for others: replay such a graph only while no other call or graph is running.
  * Per-set problems are reported in err[], not as a failed call.  (k > 128: a
  * set's CTAs wait for one another for 2 s at most; sets that time out are NaN
  * with PL_SET_TIMEDOUT, and pl_solve_host returns PL_ETIMEDOUT.)

@@ -511,8 +511,11 @@ struct MatCache {
 };
 
 struct DevState {
-  DevScratch large;    // k_large slots
+  DevScratch large;    // bisection queues, k_large slots
   DevScratch bins;     // counts / starts / cursor / perm
+  cudaEvent_t ev_shared = nullptr;  // the last call's use of large and bins (SharedScratch)
+  bool shared_used = false;
+  unsigned long long shared_stream = 0;  // cudaStreamGetId of its stream (never given to another one)
   DevScratch upload;   // pl_solve_host and drop-in staging
   DevScratch mat64;    // drop-in: the FP64 matrix as uploaded
   DevScratch mat32;    // drop-in: its FP32 conversion (MatCache)
@@ -560,6 +563,35 @@ int ensure(DevScratch& s, size_t bytes) {
   return PL_OK;
 }
 
+// Device-pointer calls return before their kernels run, and calls on different
+// streams share the scratch buffers: a call waits, on its stream, for the one before
+// if that went to another stream (256 sets of k = 16 back to back take 21.5 us with
+// and without the event; with a wait in every call 21.7).  Not while the stream is
+// captured: a captured call cannot wait for what is outside its graph.
+struct SharedScratch {
+  DevState& d;
+  cudaStream_t st;
+  bool on = false;
+  SharedScratch(DevState& d_, cudaStream_t st_) : d(d_), st(st_) {}
+  cudaError_t begin() {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(st, &cs);
+    if (e != cudaSuccess || cs != cudaStreamCaptureStatusNone) return e;
+    on = true;
+    unsigned long long id = 0;
+    e = cudaStreamGetId(st, &id);
+    if (e == cudaSuccess && !d.ev_shared) e = cudaEventCreateWithFlags(&d.ev_shared, cudaEventDisableTiming);
+    if (e == cudaSuccess && d.shared_used && d.shared_stream != id) e = cudaStreamWaitEvent(st, d.ev_shared, 0);
+    d.shared_stream = id;
+    return e;
+  }
+  cudaError_t end() {
+    if (!on) return cudaSuccess;
+    d.shared_used = true;
+    return cudaEventRecord(d.ev_shared, st);
+  }
+};
+
 int ensure_streams(DevState& d) {
   if (d.ev_fork) return PL_OK;
   PL_CU(cudaEventCreateWithFlags(&d.ev_fork, cudaEventDisableTiming));
@@ -591,10 +623,12 @@ int solve_uniform(const MatrixF32& M, const int* idx, long long nsets, int k, in
   const Variant& v = chosen_for(b, all);
   void* scratch = nullptr;
   const size_t need = v.scratch[all ? 1 : 0]();
+  SharedScratch shared(state(), st);
   if (need) {
     int rc = ensure(state().large, need);
     if (rc) return rc;
     scratch = state().large.p;
+    PL_CU(shared.begin());
   }
   LaunchFn fn = v.fn[all ? 1 : 0];
   if (all && v.few_all) {
@@ -610,6 +644,7 @@ int solve_uniform(const MatrixF32& M, const int* idx, long long nsets, int k, in
     if (LaunchFn few = few_all_fn(v, nsets)) fn = few;
   }
   PL_CU(fn(M, src, out, nsets, scratch, st, false));
+  if (need) PL_CU(shared.end());
   return PL_OK;
 }
 
@@ -727,7 +762,10 @@ int solve_csr(const MatrixF32& M, const int* idx, const long long* offsets, long
     }
     it = d.graphs.emplace(key, DevState::GraphEntry{exec}).first;
   }
+  SharedScratch shared(d, st);
+  PL_CU(shared.begin());
   PL_CU(cudaGraphLaunch(it->second.exec, st));
+  PL_CU(shared.end());
   return PL_OK;
 }
 
@@ -1234,6 +1272,9 @@ int pl_release(void) {
     s->p = nullptr;
     s->bytes = 0;
   }
+  if (d.ev_shared) cudaEventDestroy(d.ev_shared);
+  d.ev_shared = nullptr;
+  d.shared_used = false;
   if (d.timed_out) cudaFreeHost(d.timed_out);
   d.timed_out = nullptr;
   d.mc.valid = false;
