@@ -376,7 +376,7 @@ struct Variant {
 // of few sets on the register engine, two warps per set
 #define SAPT(KB, RPT, CTA, REGS, NB)                                                         \
   Variant {                                                                                    \
-    "tmemA ahead KB=" #KB " RPT=" #RPT " CTA=" #CTA " REGS=" #REGS " NB=" #NB,                 \
+    "sharedA prefetch tmem KB=" #KB " RPT=" #RPT " CTA=" #CTA " REGS=" #REGS " NB=" #NB,                 \
         {launch_sap<KB, RPT, CTA, REGS, NB>, launch_sap<KB, RPT, CTA, 255, NB, true>},          \
         {scratch_sap<KB, RPT, CTA, REGS, NB>, scratch_none}, true,                              \
         launch_reg<KB, 1, 1, 128, 3, true>                                                      \
