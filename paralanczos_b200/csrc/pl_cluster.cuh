@@ -19,9 +19,10 @@
 // needs.  No CTA barrier, no cluster barrier (whose release fence the warps
 // would wait for) and no second pass over the partials.  Measured (B200,
 // sets/s) with a cluster barrier per exchange and A_S in shared memory, then
-// with st.async, then with A_S in tensor memory: k = 384 (1,000 sets) 2.55e4,
-// 3.39e4, 3.57e4; k = 512 (600 sets) 8.7e3, 1.19e4, 1.41e4; with one CTA per
-// set k = 192 (3,000 sets) 3.06e5, 3.55e5, 4.51e5.
+// with st.async, then with A_S in tensor memory, then with no use of P's registers
+// outside the passes: k = 384 (1,000 sets) 2.55e4, 3.39e4, 3.51e4, 3.74e4; k = 512
+// (600 sets) 8.7e3, 1.19e4, 1.36e4, 1.45e4; with one CTA per set k = 192 (3,000
+// sets) 3.06e5, 3.55e5, 4.47e5, 4.56e5.
 //
 // Thread mapping inside a CTA: NTC threads; a thread holds RPT of the CTA's
 // R rows (rows ls, ls + R/RPT, ...), TPR = NTC * RPT / R threads share a row;
@@ -62,6 +63,7 @@ struct CfgC {
   static constexpr int CPT = KB / TPR;    // columns per thread (of each of its rows)
   static constexpr int NCH = CPT / 4;     // float4 chunks per thread and row
   static constexpr int NWC = NTC / 32;    // warps per CTA
+  static_assert(R <= NTC, "a thread per own row");
   static_assert(KB % CS == 0 && R % RPT == 0 && NTC % RS == 0 && KB % TPR == 0, "bad shape");
   static constexpr int CPR = TPR / RPT;  // lanes that end with a row's sum
   static constexpr int NP = (CS + CPR - 1) / CPR;  // peers such a lane sends it to
@@ -72,19 +74,22 @@ struct CfgC {
 template <int KB, int CS, int NTC>
 struct __align__(16) ClusterSmem {
   static constexpr int NPART = CS * (NTC / 32);  // one partial per warp of the set
-  // [float4 of a thread][thread]: P between the segments of the step loop (and,
-  // before the first, where one CTA mirrors its triangle of A_S)
-  float4 P[(KB / CS) * KB / 4];
+  // before the steps, where one CTA mirrors its triangle of A_S: [float4 of a
+  // thread][thread]; from then on the own rows of every step's vector: [step][row]
+  float4 own[(KB / CS) * KB / 4];
   float vb[3][KB];               // unnormalised Lanczos vectors, rotating: current, previous, next
   float yb[KB];                  // broadcast of y = A v
   float wb[KB];                  // w~, formed locally from yb
   int idx[KB];
+  float sc[KB];                  // every step's scale (v = sc * vb)
+  float diag[KB / CS];           // own diagonal elements of P, up to step `seen`
   double2 ab[KB];                // T (rank 0 reads it for the bisection)
   double part[4][NPART];         // alpha, ||w||^2, misc, index check
   double ext[2];                 // lambda_min, lambda_max
   double red[NTC / 32];          // warp partials inside the CTA (breakdown argmax)
   unsigned long long key[CS];    // breakdown argmax exchange
   unsigned long long bar[2];     // mbarriers of the y and the w exchange
+  int seen;
   int abort;                     // a bounded wait gave up, here or in a peer
   long long lost;                // the item it was on
 };
@@ -177,14 +182,12 @@ __device__ __forceinline__ float row_reduce(float (&y)[RPT], int g0) {
   return y[0];
 }
 
-enum ClusterResult { CLUSTER_DONE, CLUSTER_RESTARTED, CLUSTER_BROKE, CLUSTER_ABORT };
+enum ClusterResult { CLUSTER_DONE, CLUSTER_ABORT };
 
 // Solves one set on the cluster.
-//   DONE       its outputs are written
-//   RESTARTED  the same, and it had a breakdown (RESTART)
-//   BROKE      it had a breakdown, nothing is written (!RESTART)
-//   ABORT      a bounded wait gave up somewhere in the cluster: nothing is
-//              written, and every CTA of the cluster must end
+//   DONE   its outputs are written
+//   ABORT  a bounded wait gave up somewhere in the cluster: nothing is written,
+//          and every CTA of the cluster must end
 // A wait that gives up is a warp's answer first, then the CTA's (a vote in
 // every step, and at the end of the steps), then the cluster's: no CTA passes
 // the barrier at the end of its steps before every other one is there, and
@@ -192,14 +195,20 @@ enum ClusterResult { CLUSTER_DONE, CLUSTER_RESTARTED, CLUSTER_BROKE, CLUSTER_ABO
 // CTA writes into one that has left.  hold (tests): 1, the last CTA stays out of
 // the steps until its peers' waits have run out; 2, it gives up behind the last
 // one, when its peers have all they need.
-// RESTART: with the breakdown restart.  P then has to outlive the step loop,
-// which costs the loop 80 to 400 bytes of spills at 168 and 255 registers
-// wherever the restart stands (k = 512 1.04 -> 1.25 ms a set, k = 384 0.86 ->
-// 1.32), so a set is first solved without it, and again with it if it breaks
-// down; the two do the same arithmetic.  ph: phase parity of the exchanges,
-// kept across sets.  ta: the thread's tensor memory, read NB float4 at a
-// time.
-template <int KB, int CS, int NTC, int RPT, int NB, bool RESTART>
+// ph: phase parity of the exchanges, kept across sets.  ta: the thread's tensor
+// memory, read NB float4 at a time.
+//
+// A breakdown restarts from a row of P.  Any use of P's registers outside the two
+// passes costs the loop 80 to 400 bytes of spills at 168 and 255 registers (k = 384
+// 0.86 -> 1.32 ms a set), and solving a set again with them is twice the work, so
+// the restart forms the diagonal and the row anew, by the same operations in the
+// same order, from the vectors of the steps so far (in shared memory that the
+// steps leave idle; one float a thread and step).  660 sets of k = 384, none, each
+// second and all of them with some 39 restarts: 17.4, 19.1 and 20.7 ms (with sets that
+// break down solved twice 18.3, 35.9 and 30.7; with P at hand in every loop 23.2,
+// 24.4 and 25.5).  The loop of one CTA per set has room for P at hand (k = 192,
+// 3,000 sets: 6.6 ms, from the vectors 6.8).
+template <int KB, int CS, int NTC, int RPT, int NB>
 __device__ __forceinline__ ClusterResult cluster_solve_set(const MatrixF32& M, const int* __restrict__ S,
                                                   int k, long long set, const SetOutputs& out,
                                                   ClusterSmem<KB, CS, NTC>& sm,
@@ -277,7 +286,7 @@ __device__ __forceinline__ ClusterResult cluster_solve_set(const MatrixF32& M, c
   // ---- gather own rows of A_S into tensor memory -----------------------------
   constexpr int NF = NCH * RPT;  // float4 of a thread, (q, ch) as number ch * RPT + q
   static_assert(NF % NB == 0 && NF % 4 == 0, "whole buffers");
-  // float offset in sm.P of the CTA's element (row, col): chunk cc = col / 4 of
+  // float offset in sm.own of the CTA's element (row, col): chunk cc = col / 4 of
   // row q * RS + ls belongs to the thread of slot ls and g = cc % TPR as its
   // (q, cc / TPR)
   auto at = [](int row, int col) {
@@ -285,8 +294,8 @@ __device__ __forceinline__ ClusterResult cluster_solve_set(const MatrixF32& M, c
     const int th = (sl / RPW) * 32 + (cc % TPR) * RPW + sl % RPW;
     return (((cc / TPR * RPT + row / RS) * NTC + th) << 2) + (col & 3);
   };
-  float* __restrict__ Pf = reinterpret_cast<float*>(sm.P);
-  float4* __restrict__ my = sm.P + t;  // number i at my[i * NTC]
+  float* __restrict__ own = reinterpret_cast<float*>(sm.own);
+  [[maybe_unused]] float4* __restrict__ my = sm.own + t;  // number i at my[i * NTC]
   double fro = 0.0;
   if constexpr (CS == 1) {
     // One CTA holds all of A_S, which is symmetric: load only its upper
@@ -309,8 +318,8 @@ __device__ __forceinline__ ClusterResult cluster_solve_set(const MatrixF32& M, c
       const float e = (rr < k && c < k) ? __ldg((first ? row0 : row1) + sm.idx[c]) : 0.f;
       const double e2 = (double)e * (double)e;
       fro += (c == rr) ? e2 : 2.0 * e2;
-      Pf[at(rr, c)] = e;
-      if (c != rr) Pf[at(c, rr)] = e;
+      own[at(rr, c)] = e;
+      if (c != rr) own[at(c, rr)] = e;
     }
     __syncthreads();
 #pragma unroll 4
@@ -342,13 +351,6 @@ __device__ __forceinline__ ClusterResult cluster_solve_set(const MatrixF32& M, c
     }
   }
   tmem_st_wait();
-  if constexpr (RESTART) {  // P = I
-    for (int i = 0; i < NF; ++i) {
-      const int row = rank * R + ls + (i % RPT) * RS, c = 4 * (g0 + TPR * (i / RPT));
-      const bool rv = row < k;
-      my[i * NTC] = make_float4(rv && c == row, rv && c + 1 == row, rv && c + 2 == row, rv && c + 3 == row);
-    }
-  }
   const double fro2 = cluster_sum<KB, CS, NTC>(fro, sm, 2, cl, rank);
   const double tau2 = (32.0 * (double)kEps32) * (32.0 * (double)kEps32) * fro2;
 
@@ -367,37 +369,32 @@ __device__ __forceinline__ ClusterResult cluster_solve_set(const MatrixF32& M, c
     sm.vb[0][c] = c < k ? v0 : 0.f;
     sm.vb[1][c] = 0.f;
   }
-  if (t == 0) sm.ab[0].y = 0.0;
+  if (t == 0) {
+    sm.ab[0].y = 0.0;
+    sm.seen = 0;
+  }
   float sc = 1.f, scp = 0.f, bprev = 0.f;
   int status = 0;
   int cur = 0, prv = 1, nxt = 2;
   __syncthreads();
   TmemBuf<NB> buf[2];
+  float2 Pr[RPT][CPT / 2];
+#pragma unroll
+  for (int q = 0; q < RPT; ++q)
+#pragma unroll
+    for (int ch = 0; ch < NCH; ++ch) {  // I
+      const int c = 4 * (g0 + TPR * ch);
+      const bool rv = r[q] < k;
+      Pr[q][2 * ch] = make_float2(rv && c == r[q], rv && c + 1 == r[q]);
+      Pr[q][2 * ch + 1] = make_float2(rv && c + 2 == r[q], rv && c + 3 == r[q]);
+    }
+  [[maybe_unused]] float pd = ro < k ? 1.f : 0.f;  // (one CTA) P's diagonal element of row ro
   if (CS > 1 && hold == 1 && rank == CS - 1) {
     for (const unsigned long long t0 = globaltimer(); globaltimer() - t0 < kWaitNs + kWaitNs / 4;) __nanosleep(10000);
     goto lost;
   }
-  // Steps run in segments: a breakdown leaves the step loop, restarts the
-  // recurrence from P in shared memory and enters the loop again.
+  buf[0].load(ta, 0);
   for (int j = 0;; ++j) {
-    float2 Pr[RPT][CPT / 2];
-#pragma unroll
-    for (int q = 0; q < RPT; ++q)
-#pragma unroll
-      for (int ch = 0; ch < NCH; ++ch) {
-        if constexpr (RESTART) {
-          const float2* p2 = reinterpret_cast<const float2*>(my + (ch * RPT + q) * NTC);
-          Pr[q][2 * ch] = p2[0];
-          Pr[q][2 * ch + 1] = p2[1];
-        } else {  // I
-          const int c = 4 * (g0 + TPR * ch);
-          const bool rv = r[q] < k;
-          Pr[q][2 * ch] = make_float2(rv && c == r[q], rv && c + 1 == r[q]);
-          Pr[q][2 * ch + 1] = make_float2(rv && c + 2 == r[q], rv && c + 3 == r[q]);
-        }
-      }
-    buf[0].load(ta, 0);
-    for (;; ++j) {
     if constexpr (CS > 1) {
       if (t == 0) {
         mbar_expect(ybar, exchange_bytes<KB, CS, NTC>());
@@ -405,6 +402,7 @@ __device__ __forceinline__ ClusterResult cluster_solve_set(const MatrixF32& M, c
       }
     }
     // P -= v v^T and y = A v over the owned row slices
+    if constexpr (CS == 1) pd = fmaf(-vo * sc, sm.vb[cur][ro], pd);
     float2 ya[RPT], yb[RPT], nc[RPT];
 #pragma unroll
     for (int q = 0; q < RPT; ++q) {
@@ -484,6 +482,10 @@ __device__ __forceinline__ ClusterResult cluster_solve_set(const MatrixF32& M, c
     publish_row(sm.vb[nxt], wo, wbar);
     publish_partial(1, warp_sum(lead ? (double)wo * (double)wo : 0.0), wbar);
     buf[0].load(ta, 0);  // the next pass's first buffer
+    if constexpr (CS > 1) {  // (here, while w travels)
+      if (t < R) own[j * R + t] = sm.vb[cur][rank * R + t];
+      if (t == 0) sm.sc[j] = sc;
+    }
     const bool got_w = arrived(wbar);
 #pragma unroll
     for (int q = 0; q < RPT; ++q) v[q] = sm.vb[nxt][r[q]];
@@ -501,89 +503,100 @@ __device__ __forceinline__ ClusterResult cluster_solve_set(const MatrixF32& M, c
       goto steps_done;
     }
     if (j + 1 == k) goto steps_done;
-    if (!(b2v > tau2)) break;
-    const float bf = sqrtf((float)b2v);
-    scp = sc;
-    sc = 1.0f / bf;
-    bprev = bf;
-    vo = wo * sc;
+    if (b2v > tau2) {
+      const float bf = sqrtf((float)b2v);
+      scp = sc;
+      sc = 1.0f / bf;
+      bprev = bf;
+      vo = wo * sc;
 #pragma unroll
-    for (int q = 0; q < RPT; ++q) v[q] *= sc;
-    const int old_prv = prv;
-    prv = cur;
-    cur = nxt;
-    nxt = old_prv;
-  }
-    buf[0].ready();  // no load outlives the segment
-    if constexpr (!RESTART) {
+      for (int q = 0; q < RPT; ++q) v[q] *= sc;
+    } else {
+      // Breakdown: restart from the row of P with the largest diagonal
+      // (cluster-wide argmax, ties to the smaller row), published into vb[nxt].
+      status |= SET_BREAKDOWN;
       if constexpr (CS > 1) {
         if (__syncthreads_or(0)) goto failed;
         set_sync<CS>(cl);
         if (sm.abort) goto leave;
       }
-      return CLUSTER_BROKE;
-    }
-    // Breakdown: restart from the column of P with the largest diagonal
-    // (cluster-wide argmax, ties to the smaller row), published into vb[nxt].
-    status |= SET_BREAKDOWN;
-#pragma unroll
-    for (int q = 0; q < RPT; ++q)
-#pragma unroll
-      for (int ch = 0; ch < NCH; ++ch) {
-        float2* p2 = reinterpret_cast<float2*>(my + (ch * RPT + q) * NTC);
-        p2[0] = Pr[q][2 * ch];
-        p2[1] = Pr[q][2 * ch + 1];
+      unsigned long long kk = 0ull;
+      if constexpr (CS == 1) {
+        if (ro < k) kk = ((unsigned long long)__float_as_uint(fmaxf(pd, 0.f)) << 32) | (unsigned)(0x7fffffff - ro);
+      } else if (t < R && rank * R + t < k) {
+        const int row = rank * R + t;
+        float d = sm.seen ? sm.diag[t] : 1.f;
+#pragma unroll 8
+        for (int i = sm.seen; i <= j; ++i) {
+          const float b = own[i * R + t], c = sm.sc[i];
+          d = fmaf(-(b * c) * c, b, d);
+        }
+        sm.diag[t] = d;
+        kk = ((unsigned long long)__float_as_uint(fmaxf(d, 0.f)) << 32) | (unsigned)(0x7fffffff - row);
       }
-    if constexpr (CS > 1) {
-      if (__syncthreads_or(0)) goto failed;
-      set_sync<CS>(cl);
-      if (sm.abort) goto leave;
-    } else {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long y2 = __shfl_xor_sync(0xffffffffu, kk, o);
+        kk = y2 > kk ? y2 : kk;
+      }
+      if ((t & 31) == 0) sm.red[t >> 5] = __longlong_as_double((long long)kk);
       __syncthreads();
-    }
-    unsigned long long kk = 0ull;
-    for (int e = t; e < R && rank * R + e < k; e += NTC) {
-      const int row = rank * R + e;
-      const float d = fmaxf(Pf[at(e, row)], 0.f);
-      const unsigned long long kq = ((unsigned long long)__float_as_uint(d) << 32) | (unsigned)(0x7fffffff - row);
-      kk = kq > kk ? kq : kk;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long y2 = __shfl_xor_sync(0xffffffffu, kk, o);
-      kk = y2 > kk ? y2 : kk;
-    }
-    if ((t & 31) == 0) sm.red[t >> 5] = __longlong_as_double((long long)kk);
-    __syncthreads();
-    if (t < CS) {
-      unsigned long long m = 0;
-      for (int i = 0; i < NTC / 32; ++i) {
-        const unsigned long long y2 = (unsigned long long)__double_as_longlong(sm.red[i]);
-        m = y2 > m ? y2 : m;
+      if (t == 0) sm.seen = j + 1;
+      if (t < CS) {
+        unsigned long long m = 0;
+        for (int i = 0; i < NTC / 32; ++i) {
+          const unsigned long long y2 = (unsigned long long)__double_as_longlong(sm.red[i]);
+          m = y2 > m ? y2 : m;
+        }
+        cl.map_shared_rank(&sm, (unsigned)t)->key[rank] = m;
       }
-      cl.map_shared_rank(&sm, (unsigned)t)->key[rank] = m;
-    }
-    set_sync<CS>(cl);
-    unsigned long long best = 0;
+      set_sync<CS>(cl);
+      unsigned long long best = 0;
+      for (int q = 0; q < CS; ++q) best = sm.key[q] > best ? sm.key[q] : best;
+      const int mrow = 0x7fffffff - (int)(best & 0xffffffffu);
+      if constexpr (CS == 1) {
 #pragma unroll
-    for (int q = 0; q < CS; ++q) best = sm.key[q] > best ? sm.key[q] : best;
-    const int mrow = 0x7fffffff - (int)(best & 0xffffffffu);
-    if (mrow / R == rank) {
-      for (int e = t; e < CS * KB; e += NTC) {
-        ClusterSmem<KB, CS, NTC>* peer = CS == 1 ? &sm : cl.map_shared_rank(&sm, (unsigned)(e / KB));
-        peer->vb[nxt][e % KB] = Pf[at(mrow - rank * R, e % KB)];
+        for (int q = 0; q < RPT; ++q)
+          if (r[q] == mrow) {
+#pragma unroll
+            for (int ch = 0; ch < NCH; ++ch)
+              *reinterpret_cast<float4*>(&sm.vb[nxt][4 * (g0 + TPR * ch)]) =
+                  make_float4(Pr[q][2 * ch].x, Pr[q][2 * ch].y, Pr[q][2 * ch + 1].x, Pr[q][2 * ch + 1].y);
+          }
+      } else {
+        // row mrow of P: its owner sends the coefficients of the steps, every CTA forms
+        // its own columns' elements (one thread each) and sends them
+        if (mrow / R == rank) {
+          for (int e = t; e < CS * (j + 1); e += NTC) {
+            const int p = e / (j + 1), i = e - p * (j + 1);
+            const float b = own[i * R + mrow - rank * R], c = sm.sc[i];
+            ClusterSmem<KB, CS, NTC>* peer = cl.map_shared_rank(&sm, (unsigned)p);
+            peer->wb[i] = -(b * c) * c;
+          }
+        }
+        set_sync<CS>(cl);
+        if (t < R) {
+          float z = rank * R + t == mrow ? 1.f : 0.f;
+#pragma unroll 8
+          for (int i = 0; i <= j; ++i) z = fmaf(sm.wb[i], own[i * R + t], z);
+#pragma unroll 1
+          for (int p = 0; p < CS; ++p) {
+            ClusterSmem<KB, CS, NTC>* peer = cl.map_shared_rank(&sm, (unsigned)p);
+            peer->vb[nxt][rank * R + t] = z;
+          }
+        }
       }
-    }
-    set_sync<CS>(cl);
-    const float zo = sm.vb[nxt][ro];
-    const double zz = cluster_sum<KB, CS, NTC>(lead ? (double)zo * (double)zo : 0.0, sm, 2, cl, rank);
-    if (t == 0 && rank == 0) sm.ab[j + 1].y = 0x1p-600;  // decoupled block (see sturm_count)
-    scp = sc;
-    sc = 1.0f / sqrtf((float)zz);
-    bprev = 0.f;
-    vo = zo * sc;
+      set_sync<CS>(cl);
+      const float zo = sm.vb[nxt][ro];
+      const double zz = cluster_sum<KB, CS, NTC>(lead ? (double)zo * (double)zo : 0.0, sm, 2, cl, rank);
+      if (t == 0 && rank == 0) sm.ab[j + 1].y = 0x1p-600;  // decoupled block (see sturm_count)
+      scp = sc;
+      sc = 1.0f / sqrtf((float)zz);
+      bprev = 0.f;
+      vo = zo * sc;
 #pragma unroll
-    for (int q = 0; q < RPT; ++q) v[q] = sm.vb[nxt][r[q]] * sc;
+      for (int q = 0; q < RPT; ++q) v[q] = sm.vb[nxt][r[q]] * sc;
+    }
     const int old_prv = prv;
     prv = cur;
     cur = nxt;
@@ -631,7 +644,7 @@ steps_done:
     }
   }
   set_sync<CS>(cl);  // rank 0's reads of T precede the next set's writes
-  return (status & SET_BREAKDOWN) ? CLUSTER_RESTARTED : CLUSTER_DONE;
+  return CLUSTER_DONE;
 
 lost:  // this warp: its vote
   __syncthreads_or(1);

@@ -303,7 +303,6 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NTC, 1)
   uint32_t ph = 0;
   TmemA<KB / CS * KB / NTC, NTC, NB> am;
   am.begin();
-  bool likely_breaks = false;
   const long long nitems = item_count(src);
   const int pbase = src.perm_start ? *src.perm_start : 0;
   for (long long it = cid; it < nitems; it += ncl) {  // the same items on every rank
@@ -314,22 +313,8 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NTC, 1)
       if (rank == 0 && threadIdx.x == 0) write_failed(out, set, off, 0, SET_BAD_K);
       continue;
     }
-    ClusterResult res = CLUSTER_DONE;
-    // one CTA: the loop fits its registers with the restart (0.30 ms a set
-    // either way at k = 192, and a breakdown costs no second solve).  A set after
-    // one that broke down is likely to break down too.
-    if constexpr (CS > 1) {
-      if (!likely_breaks) {
-        res = cluster_solve_set<KB, CS, NTC, RPT, NB, false>(M, src.idx + off, k, set, out, sm, cl, rank, ph, am.ta,
-                                                             hold);
-        likely_breaks = res == CLUSTER_BROKE;
-      }
-    }
-    if (CS == 1 || likely_breaks) {
-      res = cluster_solve_set<KB, CS, NTC, RPT, NB, true>(M, src.idx + off, k, set, out, sm, cl, rank, ph, am.ta,
-                                                          hold);
-      likely_breaks = res == CLUSTER_RESTARTED;
-    }
+    const ClusterResult res =
+        cluster_solve_set<KB, CS, NTC, RPT, NB>(M, src.idx + off, k, set, out, sm, cl, rank, ph, am.ta, hold);
     if (CS > 1 && res == CLUSTER_ABORT) {
       if (threadIdx.x == 0) sm.lost = it;
       break;
