@@ -19,7 +19,7 @@ constexpr int kMaxPieces = 2048;          // request pieces one wave can hold
 // waves: a misestimate changes wave lengths, never results.
 __host__ __device__ inline double set_cost_us(int k) {
   const int kb[11] = {8, 16, 32, 48, 64, 96, 128, 192, 256, 384, 512};
-  const double tb[11] = {0.001, 0.003, 0.0145, 0.045, 0.089, 0.334, 0.74, 3.2, 6.0, 38.9, 115.0};
+  const double tb[11] = {0.00058, 0.0027, 0.0119, 0.0392, 0.0662, 0.247, 0.569, 2.14, 5.57, 27.0, 69.2};
   for (int b = 0; b < 11; ++b) {
     if (k <= kb[b]) {
       const double x = (double)k / kb[b];
