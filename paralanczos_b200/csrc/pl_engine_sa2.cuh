@@ -65,7 +65,7 @@ template <int KB, int RPT, int NB>
 __device__ __forceinline__ int solve_set_sa2(const MatrixF32& M, const int* __restrict__ S, int k,
                                               long long set, long long off, const SetOutputs& out,
                                               SA2Smem<KB, RPT>& sm, const Grp<CfgSA2<KB, RPT>::NT>& g,
-                                              uint32_t ta = 0) {
+                                              uint32_t ta) {
   using C = CfgSA2<KB, RPT>;
   constexpr int NT = C::NT, NW = C::NW, NR = C::NR, TPR = C::TPR, NCHT = C::NCHT;
   const int t = g.t;
@@ -183,14 +183,12 @@ __device__ __forceinline__ int solve_set_sa2(const MatrixF32& M, const int* __re
   // the thread's row parts of A_S into tensor memory, and the first buffer of
   // the first pass
   constexpr int NF = NCHT * RPT;
-  static_assert(NB == 0 || NF % (NB ? NB : 1) == 0, "whole buffers");
-  [[maybe_unused]] TmemBuf<NB ? NB : 4> buf[2];
-  if constexpr (NB > 0) {
+  static_assert(NF % NB == 0, "whole buffers");
+  TmemBuf<NB> buf[2];
 #pragma unroll
-    for (int i = 0; i < NF; ++i) tmem_st4(ta, 4 * i, my[((i % RPT) * NCHT + i / RPT) * NT]);
-    tmem_st_wait();
-    buf[0].load(ta, 0);
-  }
+  for (int i = 0; i < NF; ++i) tmem_st4(ta, 4 * i, my[((i % RPT) * NCHT + i / RPT) * NT]);
+  tmem_st_wait();
+  buf[0].load(ta, 0);
 
   for (int j = 0; j < k; ++j) {
     // P -= v v^T and y = A v over the owned chunks
@@ -208,17 +206,12 @@ __device__ __forceinline__ int solve_set_sa2(const MatrixF32& M, const int* __re
       const float2 b01 = make_float2(b4.x, b4.y), b23 = make_float2(b4.z, b4.w);
 #pragma unroll
       for (int q = 0; q < RPT; ++q) {
-        float4 a4;
-        if constexpr (NB > 0) {
-          const int i = ch * RPT + q, bi = i / NB;
-          if (i % NB == 0) {
-            buf[bi & 1].ready();
-            if ((bi + 1) * NB < NF) buf[(bi + 1) & 1].load(ta, 4 * NB * (bi + 1));
-          }
-          a4 = buf[bi & 1].f4(i % NB);
-        } else {
-          a4 = my[(q * NCHT + ch) * NT];
+        const int i = ch * RPT + q, bi = i / NB;
+        if (i % NB == 0) {
+          buf[bi & 1].ready();
+          if ((bi + 1) * NB < NF) buf[(bi + 1) & 1].load(ta, 4 * NB * (bi + 1));
         }
+        const float4 a4 = buf[bi & 1].f4(i % NB);
         Pr[q][2 * ch] = __ffma2_rn(ncoef[q], b01, Pr[q][2 * ch]);
         Pr[q][2 * ch + 1] = __ffma2_rn(ncoef[q], b23, Pr[q][2 * ch + 1]);
         ya[q] = __ffma2_rn(make_float2(a4.x, a4.y), b01, ya[q]);
@@ -274,7 +267,7 @@ __device__ __forceinline__ int solve_set_sa2(const MatrixF32& M, const int* __re
         sm.vb[rs + q * NR] = ww[q];  // published by the barrier inside group_sum
       }
     }
-    if constexpr (NB > 0) buf[0].load(ta, 0);  // the next pass's first buffer
+    buf[0].load(ta, 0);  // the next pass's first buffer
     const double b2v = group_sum<NT, NW>(bp, g, sm.red[1]);
     if (t == 0) {
       sm.ab[j].x = alpha;
@@ -353,7 +346,7 @@ __device__ __forceinline__ int solve_set_sa2(const MatrixF32& M, const int* __re
       for (int q = 0; q < RPT; ++q) v[q] = z[q] * inv;
     }
   }
-  if constexpr (NB > 0) buf[0].ready();  // no load outlives the set
+  buf[0].ready();  // no load outlives the set
   g.sync();  // T visible to every thread
   return status;
 }

@@ -174,9 +174,9 @@ __global__ void __maxnreg__(REGS) k_sa_solve_p(MatrixF32 M, SetSource src, SetOu
 
 // ---------------------------------------------------------------------------
 // Batched form, shared-A engine with two threads per row (pl_engine_sa2.cuh),
-// extremes only: persistent, A_S in dynamic shared memory, P in registers.
+// extremes only: persistent, A_S in tensor memory, P in registers.
 // ---------------------------------------------------------------------------
-template <int KB, int CTA, int MINB, int RPT = 2, int NB = 0>
+template <int KB, int CTA, int MINB, int RPT, int NB>
 __global__ void __launch_bounds__(CTA, MINB)
     k_sa2_solve(MatrixF32 M, SetSource src, SetOutputs out, double2* __restrict__ qbuf) {
   using C = CfgSA2<KB, RPT>;
