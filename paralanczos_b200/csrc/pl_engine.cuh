@@ -41,14 +41,23 @@ struct Cfg {
   static_assert(TPR == 1 || TPR == 2, "TPR must be 1 or 2");
 };
 
+// One value per row (SAME_SUMS in solve_set), only where it is used: 16 bytes
+// more in the k <= 16 group put the four groups of a warp on the same banks
+// (512 bytes a group; all eigenvalues at k = 16, 50,000 sets: 249 -> 258 us).
+template <bool USED>
+struct RowSums {
+  double row[2][64];
+};
+template <>
+struct RowSums<false> {};
+
 template <int KB, int NW>
-struct __align__(16) GroupSmem {
+struct __align__(16) GroupSmem : RowSums<KB == 64 && NW == 2> {
   float vb[KB];         // broadcast of the (unnormalised) next Lanczos vector
   float wb[KB];         // broadcast of the three-term residual w~
   int idx[KB];          // the set's indices
   double2 ab[KB];       // T: ab[i] = {alpha_i, beta_i^2}, beta_i couples rows i-1, i
   double red[6][NW];    // cross-warp partials (slots 4/5: lambda_min/max hand-off)
-  double row[2][KB == 64 && NW == 2 ? 64 : 1];  // one value per row (SAME_SUMS)
 };
 
 template <int NT>
