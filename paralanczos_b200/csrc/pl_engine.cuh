@@ -204,12 +204,13 @@ __device__ __forceinline__ void write_failed(const SetOutputs& out, long long se
     for (int m = 0; m < k; ++m) out.eig[off + m] = nan;
 }
 
-// Solve one set with the calling group.  S: the set's k indices (global).
+// Solve one set with the calling group.  S: the set's k indices (global).  one_k:
+// the call's sets all have this k.
 template <int KB, int RPT, int TPR, bool ALL>
 __device__ __forceinline__ int solve_set(const MatrixF32& M, const int* __restrict__ S, int k,
                                           long long set, long long off, const SetOutputs& out,
                                           GroupSmem<KB, Cfg<KB, RPT, TPR>::NW>& sm,
-                                          const Grp<Cfg<KB, RPT, TPR>::NT>& g) {
+                                          const Grp<Cfg<KB, RPT, TPR>::NT>& g, bool one_k) {
   using C = Cfg<KB, RPT, TPR>;
   // All eigenvalues at 48 < k <= 64: calls of few sets run here, with two warps
   // per set, calls of many on solve_set_sa with one, and a set's results do not
@@ -497,9 +498,14 @@ __device__ __forceinline__ int solve_set(const MatrixF32& M, const int* __restri
     double prod = 1.0;
     // all of a thread's eigenvalues at once: their chains overlap
     constexpr int EV = (KB + NT - 1) / NT;
+    // k = 9 and 13 count their odd row by itself, cheaper than with the three more that fill
+    // T up (50,000 sets of k = 9 182 -> 171 us, of 13 234 -> 225), unless the warp's groups
+    // differ in k (k = 9 .. 16 mixed, 100,000 sets 616 -> 649); at k = 5 it is dearer (59 ->
+    // 73), and from k = 17 on it is the same or dearer.  Up to 16 rows need no rescaling.
+    const int rows = KB == 16 && one_k && (k & 3) == 1 ? k : (k + 3) & ~3;
     for (int m0 = t; m0 < k; m0 += EV * NT) {
       double lam[EV];
-      bisect_indices<(KB == 48 || KB == 64 ? 16 : 8), EV>(sm.ab, (k + 3) & ~3, m0, NT, glo, ghi, R, lam);
+      bisect_indices<(KB == 48 || KB == 64 ? 16 : 8), EV, (KB > 16 ? 16 : 0)>(sm.ab, rows, m0, NT, glo, ghi, R, lam);
 #pragma unroll
       for (int v = 0; v < EV; ++v) {
         const int m = m0 + v * NT;

@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(CTA, MINB)
     if constexpr (!ALL) {
       if (g.t == 0) qmeta[gic][nq] = QueueMeta{set, k, 0};
     }
-    const int st = solve_set<KB, RPT, TPR, ALL>(M, src.idx + off, k, set, off, out, smem[gic], g);
+    const int st = solve_set<KB, RPT, TPR, ALL>(M, src.idx + off, k, set, off, out, smem[gic], g, !src.offsets);
     if constexpr (!ALL) {
       if (st >= 0) {
         const int kq = (qmeta[gic][nq].k + 3) & ~3;  // with the rows that fill T up

@@ -72,7 +72,7 @@ __device__ __forceinline__ void sturm_rows(const double2* t, double x, double& p
 // have no odd rows at the end (one at a time they cost 60 to 100 cycles each).
 __device__ __forceinline__ double2 sturm_pad_row(double fro) { return make_double2(4.0 * fro + 0x1p-290, 0.0); }
 
-// N rows from row i on for each x, rescaled every RES rows.
+// N rows from row i on for each x, rescaled every RES rows (0: never).
 template <int N, int E, bool FIRST, int RES>
 __device__ __forceinline__ void sturm_block(const double2* __restrict__ ab, int stride, int i, const double (&x)[E],
                                             double (&p0)[E], double (&p1)[E], unsigned (&sp)[E], int (&cnt)[E]) {
@@ -81,7 +81,7 @@ __device__ __forceinline__ void sturm_block(const double2* __restrict__ ab, int 
   for (int u = 0; u < N; ++u) t[u] = ab[(size_t)(i + u) * stride];
 #pragma unroll
   for (int e = 0; e < E; ++e) {
-    if (!FIRST && (i & (RES - 1)) == 0) sturm_rescale(p0[e], p1[e]);
+    if (RES > 0 && !FIRST && (i & (RES - 1)) == 0) sturm_rescale(p0[e], p1[e]);
     sturm_rows<N, FIRST>(t, x[e], p0[e], p1[e], sp[e], cnt[e]);
   }
 }
@@ -130,7 +130,7 @@ __device__ __forceinline__ void sturm_counts(const double2* __restrict__ ab, int
     const double2 t = ab[(size_t)i * stride];
 #pragma unroll
     for (int e = 0; e < E; ++e) {
-      if (i > 0 && (i & (RES - 1)) == 0) sturm_rescale(p0[e], p1[e]);
+      if (RES > 0 && i > 0 && (i & (RES - 1)) == 0) sturm_rescale(p0[e], p1[e]);
       const double p2 = fma(t.x - x[e], p1[e], i > 0 ? -t.y * p0[e] : 0.0);
       const unsigned s2 = (unsigned)__double2hiint(p2) >> 31;
       cnt[e] += (int)(s2 ^ sp[e]);
@@ -267,7 +267,7 @@ __device__ __forceinline__ double multisect_warp(const double2* __restrict__ ab,
 
 // Eigenvalues number m, m + step, ... (E of them, 0-based, ascending; numbers
 // >= k are left alone) by R rounds of plain bisection, side by side.
-template <int U, int E>
+template <int U, int E, int RES = 16>
 __device__ __forceinline__ void bisect_indices(const double2* __restrict__ ab, int k, int m, int step,
                                                double lo, double hi, int R, double (&lam)[E]) {
   double a[E], b[E];
@@ -281,7 +281,7 @@ __device__ __forceinline__ void bisect_indices(const double2* __restrict__ ab, i
     int cnt[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) x[e] = 0.5 * (a[e] + b[e]);
-    sturm_counts<U, E>(ab, 1, k, x, cnt);
+    sturm_counts<U, E, RES>(ab, 1, k, x, cnt);
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       if (cnt[e] >= m + e * step + 1) b[e] = x[e]; else a[e] = x[e];
