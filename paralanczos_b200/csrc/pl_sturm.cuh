@@ -12,14 +12,13 @@
 
 namespace pl {
 
-// Power-of-two rescaling of the last two minors by p1's exponent, or by p0's
-// where p1 is zero or subnormal: exact, keeps signs and ratios.  (Without a
+// Power-of-two rescaling of the last two minors by the larger one's exponent
+// (where p1 vanishes it is p0's): exact, keeps signs and ratios.  (Without a
 // branch: a taken-or-not one costs as much as ten rows.)
 __device__ __forceinline__ void sturm_rescale(double& p0, double& p1) {
-  const int f1 = (__double2hiint(p1) >> 20) & 0x7ff;  // |p1| = m * 2^(f1 - 1023), m in [1, 2)
-  const int f = f1 < 2 ? (__double2hiint(p0) >> 20) & 0x7ff : f1;
-  const int c = f < 1 ? 1 : (f > 2043 ? 2043 : f);
-  const double s = __hiloint2double((2046 - c) << 20, 0);  // 2^(1023 - c)
+  constexpr int ONE = 1 << 20;  // an exponent of 1 in a high word
+  const int f = max(__double2hiint(p0) & 2047 * ONE, __double2hiint(p1) & 2047 * ONE);
+  const double s = __hiloint2double(2046 * ONE - min(f, 2045 * ONE), 0);  // 2^(1023 - f / ONE)
   p0 *= s;
   p1 *= s;
 }
