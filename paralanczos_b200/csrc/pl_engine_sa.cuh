@@ -151,15 +151,12 @@ __device__ __forceinline__ int solve_set_sa(const MatrixF32& M, const int* __res
   // (as in solve_set, whose two warps hold one row per thread: the sums of rows
   // t and of rows t + 32 one by one, then added)
   constexpr bool SAME_SUMS = ALL && KB == 64 && RPT == 2;
-  const auto row_sum = [&](double (&x)[RPT], double* red) -> double {
-    if constexpr (SAME_SUMS) {
+  constexpr int NS = SAME_SUMS ? RPT : 1;  // FP64 sums of a thread: row q adds to sum q % NS
+  const auto row_sum = [&](double (&x)[NS], double* red) -> double {
+    if constexpr (SAME_SUMS)
       return warp_sum(x[0]) + warp_sum(x[1]);
-    } else {
-      double s = 0.0;
-#pragma unroll
-      for (int q = 0; q < RPT; ++q) s += x[q];
-      return group_sum<NT, NW>(s, g, red);
-    }
+    else
+      return group_sum<NT, NW>(x[0], g, red);
   };
   const int t = g.t;
   if constexpr (PF) {
@@ -373,11 +370,11 @@ __device__ __forceinline__ int solve_set_sa(const MatrixF32& M, const int* __res
       }
     }
     float yy[RPT];
-    double ap[RPT];  // (products of two floats: exact)
+    double ap[NS] = {};
 #pragma unroll
     for (int q = 0; q < RPT; ++q) {
       yy[q] = ((ya[q].x + ya[q].y) + (yb[q].x + yb[q].y)) * sc;
-      ap[q] = (double)v[q] * (double)yy[q];
+      ap[q % NS] = fma((double)v[q], (double)yy[q], ap[q % NS]);
     }
     const double alpha = row_sum(ap, sm.red[0]);
     const float af = (float)alpha;
@@ -408,11 +405,11 @@ __device__ __forceinline__ int solve_set_sa(const MatrixF32& M, const int* __res
       }
     }
     float ww[RPT];
-    double bp[RPT];
+    double bp[NS] = {};
 #pragma unroll
     for (int q = 0; q < RPT; ++q) {
       ww[q] = (wa[q].x + wa[q].y) + (wc[q].x + wc[q].y);
-      bp[q] = (double)ww[q] * (double)ww[q];
+      bp[q % NS] = fma((double)ww[q], (double)ww[q], bp[q % NS]);
       sm.vb[t + q * NT] = ww[q];  // published by the sync below
     }
     if constexpr (NB > 0) buf[0].load(ta, 0);  // the next pass's first buffer
@@ -470,12 +467,12 @@ __device__ __forceinline__ int solve_set_sa(const MatrixF32& M, const int* __res
           }
         }
       g.sync();
-      double zp[RPT];
+      double zp[NS] = {};
       float z[RPT];
 #pragma unroll
       for (int q = 0; q < RPT; ++q) {
         z[q] = sm.vb[t + q * NT];
-        zp[q] = (double)z[q] * (double)z[q];
+        zp[q % NS] += (double)z[q] * (double)z[q];
       }
       const double zz = row_sum(zp, sm.red[1]);
       if (t == 0) sm.ab[j + 1].y = 0x1p-600;  // decoupled block (see sturm_count)
